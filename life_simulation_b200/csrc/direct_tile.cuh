@@ -112,6 +112,7 @@ __device__ __forceinline__ void direct_tile(const float* __restrict__ src, float
                                             const CUtensorMap* tmap, int* err) {
     extern __shared__ __align__(128) float smem[];
     __shared__ __align__(8) uint64_t tma_bar;
+    __shared__ GrowthExtras ex;  // the substep's noise, jitter and injection values
     const int TP = tile_pitch(TW, g.xp);       // tile pitch (floats), 4 modulo 8
     const int TR = TH + 2 * g.r;               // tile rows
     float* tile = smem;                        // [TR][TP]
@@ -126,6 +127,7 @@ __device__ __forceinline__ void direct_tile(const float* __restrict__ src, float
     const int grp = S > 1 ? tid / NT0 : 0;
     const int lt = tid - grp * NT0;
 
+    growth_extras_init(ex, p);
     // Stage the halo tile: tile[r][c] = A[(y0 - R + r) mod H][(x0 - XP + c) mod W].
     // A box inside the field is one TMA load (its TR x TP layout is the
     // tile's); a box that wraps around the torus is loaded element by element.
@@ -287,17 +289,21 @@ __device__ __forceinline__ void direct_tile(const float* __restrict__ src, float
         const int gy = y0 + ty + o;
         if (gy >= H) return;
         const float* arow = tile + (ty + o + g.r) * TP + ox + g.xp;
+        const uint32_t jrow = rand_row(uint32_t(gy), ex.jitter_base);
+        float v[OX];
 #pragma unroll
         for (int j = 0; j < OX; ++j) {
-            const int gx = x0 + ox + j;
-            if (gx >= W) break;
-            const float A = arow[j];
-            const float muJ = mu_jitter_shift(p, uint32_t(gx), uint32_t(gy));
+            const uint32_t gx = uint32_t(x0 + ox + j);
+            const float muJ = p.mu_jitter > 0.0f ? mu_jitter_shift(p, gx, jrow) : 0.0f;
             GrowthAcc ga;
 #pragma unroll
             for (int k = 0; k < NK; ++k) ga.add(p.weight[k], bell(acc[o][k][j], p.mu[k] + muJ, p.sigma[k]));
-            dst[size_t(gy) * W + gx] = growth_finish(p, A, ga, uint32_t(gx), uint32_t(gy));
+            v[j] = growth_euler(p, arow[j], ga.weighted, ga.std_sum);
         }
+        noise_inject_clip(p, ex, v, uint32_t(x0 + ox), uint32_t(gy));
+#pragma unroll
+        for (int j = 0; j < OX; ++j)
+            if (x0 + ox + j < W) dst[size_t(gy) * W + x0 + ox + j] = v[j];
     }
 }
 

@@ -236,8 +236,6 @@ __device__ __noinline__ void row_item(const SpectralWorld& sw, int y0, const flo
     const int H = int(p.height), nk = sw.nk;
     const int rows = min(RB, H - y0);
     const bool asym = p.growth_mode == 1u;
-    const bool jitter = p.mu_jitter > 0.0f;
-    const bool extras = p.noise_amount > 0.0f || p.inject_amount > 0.0f;
     const float dt = p.dt, sum_w = p.sum_weights;
     const bool sw_ok = sum_w > 1e-6f;
     if (nk > 0) stage_rows<M, RB, kPT, PITCH>(sU, U, H, y0, rows);
@@ -279,10 +277,9 @@ __device__ __noinline__ void row_item(const SpectralWorld& sw, int y0, const flo
             for (int t = 0; t < RC; ++t) z[t] = X[bi[it] * PITCH + IL::in(jj[it], t)];
             IL::template twiddle<true>(z, jj[it], twi);
             Dft<RC, true>::run(z);
-            const uint32_t gy = uint32_t(y0 + bi[it]);
 #pragma unroll
             for (int t = 0; t < RC; ++t) {
-                const float2 c = gp.term(z[t], p, jitter, uint32_t(2 * (jj[it] + t * NRC)), gy);
+                const float2 c = gp.term(z[t]);
                 acc[it][t] = kk == 0 ? c : __fadd2_rn(acc[it][t], c);
             }
         }
@@ -303,13 +300,12 @@ __device__ __noinline__ void row_item(const SpectralWorld& sw, int y0, const flo
                 za[it][t] = a;
                 continue;
             }
-            const auto finish = [&](float A, float s, uint32_t gx) {
-                if (extras) return growth_finish_call(p, A, s, s, gx, uint32_t(gy));
+            // A batch's worlds have no noise, mu jitter or injection.
+            const auto finish = [&](float A, float s) {
                 const float A2 = asym ? A + dt * ((sw_ok ? s / sum_w : A) - A) : A + dt * s;
                 return fminf(fmaxf(A2, 0.0f), 1.0f);
             };
-            const float2 r = make_float2(finish(a.x, acc[it][t].x, uint32_t(2 * n)),
-                                         finish(a.y, acc[it][t].y, uint32_t(2 * n + 1)));
+            const float2 r = make_float2(finish(a.x, acc[it][t].x), finish(a.y, acc[it][t].y));
             *reinterpret_cast<float2*>(A_out + size_t(gy) * W + 2 * n) = r;
             za[it][t] = r;
         }

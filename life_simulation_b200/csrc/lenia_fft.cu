@@ -153,9 +153,12 @@ __global__ void row_c2r_growth_kernel(FftGeometry g, const float2* __restrict__ 
     float2* ba = twr + (M + 1);
     float2* bb = ba + RB * M;
     float* acc = reinterpret_cast<float*>(bb + RB * M);  // [RB][W]
+    __shared__ GrowthExtras ex;
     load_table(tw, g.tw_row, M);
     load_table(twr, g.tw_r2c, M + 1);
+    growth_extras_init(ex, p);  // visible after the first loaded rows' barrier
     const bool asym = p.growth_mode == 1u;
+    const bool jitter = p.mu_jitter > 0.0f;
     for (int y0 = blockIdx.x * RB; y0 < H; y0 += gridDim.x * RB) {
         const int rows = min(RB, H - y0);
         for (int kk = 0; kk < g.nk; ++kk) {
@@ -191,8 +194,8 @@ __global__ void row_c2r_growth_kernel(FftGeometry g, const float2* __restrict__ 
                 const float2 u = z[q];
                 const uint32_t gy = uint32_t(y0 + r);
                 float* ar = acc + r * W + 2 * n;
-                const float m0 = mu + mu_jitter_shift(p, uint32_t(2 * n), gy);
-                const float m1 = mu + mu_jitter_shift(p, uint32_t(2 * n + 1), gy);
+                const float2 j = jitter ? mu_jitter_pair(p, ex, uint32_t(2 * n), gy) : make_float2(0.0f, 0.0f);
+                const float m0 = mu + j.x, m1 = mu + j.y;
                 const float bl0 = bell(u.x, m0, sigma), bl1 = bell(u.y, m1, sigma);
                 const float c0 = asym ? h * bl0 : h * (2.0f * bl0 - 1.0f);
                 const float c1 = asym ? h * bl1 : h * (2.0f * bl1 - 1.0f);
@@ -207,15 +210,14 @@ __global__ void row_c2r_growth_kernel(FftGeometry g, const float2* __restrict__ 
             __syncthreads();
         }
         float* af = reinterpret_cast<float*>(ba);  // A' staged as row pairs
-        for (int q = threadIdx.x; q < rows * W; q += blockDim.x) {
-            const int r = q / W, x = q - r * W;
-            const size_t gi = size_t(y0 + r) * W + x;
-            GrowthAcc ga;
-            ga.weighted = acc[q];
-            ga.std_sum = acc[q];
-            const float a2 = growth_finish(p, __ldg(A + gi), ga, uint32_t(x), uint32_t(y0 + r));
-            A_out[gi] = a2;
-            af[q] = a2;
+        for (int q = threadIdx.x; q < rows * M; q += blockDim.x) {
+            const int r = q / M, n = q - r * M;
+            const size_t gi = size_t(y0 + r) * W + 2 * n;
+            const float2 a0 = __ldg(reinterpret_cast<const float2*>(A + gi));
+            const float2 sum = *reinterpret_cast<const float2*>(acc + 2 * q);
+            const float2 a2 = growth_finish_pair(p, ex, a0, sum, uint32_t(2 * n), uint32_t(y0 + r));
+            *reinterpret_cast<float2*>(A_out + gi) = a2;
+            *reinterpret_cast<float2*>(af + 2 * q) = a2;
         }
         __syncthreads();
         if (S_next) {

@@ -279,6 +279,7 @@ __global__ void __launch_bounds__(RowK<PI, RB, SPLIT>::T,
     constexpr int M = K::M, W = 2 * M, T = K::T, PITCH = K::PITCH, RC = K::RC, NRC = K::NRC;
     extern __shared__ __align__(16) float2 sm[];
     __shared__ SpectralWorld sw;  // this CTA's world
+    __shared__ GrowthExtras ex;   // its substep's noise, jitter and injection values
     float2* twr = sm;
     float2* twi = twr + (M + 1);
     float2* twf = twi + PI::tw_size();
@@ -306,6 +307,7 @@ __global__ void __launch_bounds__(RowK<PI, RB, SPLIT>::T,
     // The Euler step's parameters in registers (the rare noise / injection
     // path reads them from the shared block out of line).
     const bool extras = p.noise_amount > 0.0f || p.inject_amount > 0.0f;
+    if (extras || jitter) growth_extras_init(ex, p);  // visible after the first staged item's barrier
     const float dt = p.dt, sum_w = p.sum_weights;
     const bool sw_ok = sum_w > 1e-6f;
     // Item idx of a row group: the rows of U_idx for idx < nk, else of A.
@@ -380,7 +382,8 @@ __global__ void __launch_bounds__(RowK<PI, RB, SPLIT>::T,
                 }
 #pragma unroll
                 for (int t = 0; t < RC; ++t) {
-                    const float2 c = gp.term(z[t], p, jitter, uint32_t(2 * (jj[it] + t * NRC)), gy);
+                    const float2 c = jitter ? gp.term(z[t], mu_jitter_pair(p, ex, uint32_t(2 * (jj[it] + t * NRC)), gy))
+                                            : gp.term(z[t]);
                     acc[it][t] = kk == 0 ? c : __fadd2_rn(acc[it][t], c);
                 }
             }
@@ -415,14 +418,14 @@ __global__ void __launch_bounds__(RowK<PI, RB, SPLIT>::T,
                     za[it][t] = a;
                     continue;
                 }
-                // growth_finish_lean with the parameters in registers.
-                const auto finish = [&](float A, float s, uint32_t gx) {
-                    if (extras) return growth_finish_call(p, A, s, s, gx, uint32_t(gy));
+                // The common case (no noise, no injection) inline, its
+                // parameters in registers.
+                const auto finish = [&](float A, float s) {
                     const float A2 = asym ? A + dt * ((sw_ok ? s / sum_w : A) - A) : A + dt * s;
                     return fminf(fmaxf(A2, 0.0f), 1.0f);
                 };
-                const float2 r = make_float2(finish(a.x, acc[it][t].x, uint32_t(2 * n)),
-                                             finish(a.y, acc[it][t].y, uint32_t(2 * n + 1)));
+                const float2 r = extras ? growth_finish_pair(p, ex, a, acc[it][t], uint32_t(2 * n), uint32_t(gy))
+                                        : make_float2(finish(a.x, acc[it][t].x), finish(a.y, acc[it][t].y));
                 *reinterpret_cast<float2*>(A_out + size_t(gy) * W + 2 * n) = r;
                 if constexpr (CM) palette_pair(sw.cm, r, sw.rgba + size_t(gy) * W + 2 * n);
                 za[it][t] = r;
