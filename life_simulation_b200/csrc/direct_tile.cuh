@@ -284,21 +284,30 @@ __device__ __forceinline__ void direct_tile(const float* __restrict__ src, float
 #pragma unroll
                 for (int j = 0; j < OX; ++j) acc[0][k][j] += part[(((q - 1) * NK + k) * NT0 + lt) * OX + j];
     }
+    const EulerStep euler(p);
 #pragma unroll
     for (int o = 0; o < OY; ++o) {
         const int gy = y0 + ty + o;
         if (gy >= H) return;
         const float* arow = tile + (ty + o + g.r) * TP + ox + g.xp;
-        const uint32_t jrow = rand_row(uint32_t(gy), ex.jitter_base);
+        float2 sum[OX / 2];  // growth sums of pixel pairs
+#pragma unroll
+        for (int k = 0; k < NK; ++k) {
+            const GrowthPair gp(p.mu[k], 1.0f / p.sigma[k], p.weight[k], euler.asym);
+#pragma unroll
+            for (int j = 0; j < OX / 2; ++j) {
+                const float2 u = make_float2(acc[o][k][2 * j], acc[o][k][2 * j + 1]);
+                const float2 c = gp.term_near(
+                    u, p.mu_jitter > 0.0f ? mu_jitter_pair(p, ex, uint32_t(x0 + ox + 2 * j), uint32_t(gy))
+                                          : make_float2(0.0f, 0.0f));
+                sum[j] = k == 0 ? c : __fadd2_rn(sum[j], c);
+            }
+        }
         float v[OX];
 #pragma unroll
-        for (int j = 0; j < OX; ++j) {
-            const uint32_t gx = uint32_t(x0 + ox + j);
-            const float muJ = p.mu_jitter > 0.0f ? mu_jitter_shift(p, gx, jrow) : 0.0f;
-            GrowthAcc ga;
-#pragma unroll
-            for (int k = 0; k < NK; ++k) ga.add(p.weight[k], bell(acc[o][k][j], p.mu[k] + muJ, p.sigma[k]));
-            v[j] = growth_euler(p, arow[j], ga.weighted, ga.std_sum);
+        for (int j = 0; j < OX / 2; ++j) {
+            v[2 * j] = euler(arow[2 * j], sum[j].x);
+            v[2 * j + 1] = euler(arow[2 * j + 1], sum[j].y);
         }
         noise_inject_clip(p, ex, v, uint32_t(x0 + ox), uint32_t(gy));
 #pragma unroll

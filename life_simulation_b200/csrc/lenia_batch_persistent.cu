@@ -236,8 +236,7 @@ __device__ __noinline__ void row_item(const SpectralWorld& sw, int y0, const flo
     const int H = int(p.height), nk = sw.nk;
     const int rows = min(RB, H - y0);
     const bool asym = p.growth_mode == 1u;
-    const float dt = p.dt, sum_w = p.sum_weights;
-    const bool sw_ok = sum_w > 1e-6f;
+    const EulerStep euler(p);
     if (nk > 0) stage_rows<M, RB, kPT, PITCH>(sU, U, H, y0, rows);
     cp_async_commit();
     stage_field_rows<M, RB, kPT, PITCH>(sA, sw.A, y0, rows);
@@ -301,11 +300,8 @@ __device__ __noinline__ void row_item(const SpectralWorld& sw, int y0, const flo
                 continue;
             }
             // A batch's worlds have no noise, mu jitter or injection.
-            const auto finish = [&](float A, float s) {
-                const float A2 = asym ? A + dt * ((sw_ok ? s / sum_w : A) - A) : A + dt * s;
-                return fminf(fmaxf(A2, 0.0f), 1.0f);
-            };
-            const float2 r = make_float2(finish(a.x, acc[it][t].x), finish(a.y, acc[it][t].y));
+            const float2 r = make_float2(fminf(fmaxf(euler(a.x, acc[it][t].x), 0.0f), 1.0f),
+                                         fminf(fmaxf(euler(a.y, acc[it][t].y), 0.0f), 1.0f));
             *reinterpret_cast<float2*>(A_out + size_t(gy) * W + 2 * n) = r;
             za[it][t] = r;
         }

@@ -65,17 +65,13 @@ __device__ __forceinline__ float mu_jitter_shift(const StepParams& p, uint32_t g
     return (rand01_row(gx, row) - 0.5f) * p.mu_jitter * 0.05f;
 }
 
-// bell(u; mu, sigma) = exp(-0.5 t^2), t = (u - mu) / sigma (Lenia.metal:156-159).
-__device__ __forceinline__ float bell(float u, float mu, float sigma) {
-    float t = (u - mu) / sigma;
-    return expf(-0.5f * t * t);
-}
-
-// The same bell with a precomputed 1/sigma and one hardware base-2
-// exponential: exp(-0.5 t^2) = 2^(-0.5 log2(e) t^2). ex2.approx.ftz has a
-// relative error below 2^-22 (negligible against the FP32 FFT's rounding),
-// and it replaces an IEEE division and the full-range expf sequence; used on
-// the spectral path, where the growth map is a large share of the row pass.
+// bell(u; mu, sigma) = exp(-0.5 t^2), t = (u - mu) / sigma (Lenia.metal:156-159)
+// with a precomputed 1/sigma and one hardware base-2 exponential: 2^(-0.5
+// log2(e) t^2). ex2.approx.ftz has a relative error below 2^-22 (dt times that
+// reaches A, under A's own rounding), and it replaces an IEEE division and the
+// full-range expf sequence: on the direct path these were about 60 of the
+// epilogue's 127 instructions a pixel.
+//
 // 2^x by the SFU's approximate base-2 exponential (relative error < 2^-22,
 // subnormal results flushed to zero).
 __device__ __forceinline__ float ex2_fast(float x) {
@@ -84,7 +80,7 @@ __device__ __forceinline__ float ex2_fast(float x) {
     return r;
 }
 
-// One kernel's growth terms at a pixel pair of the spectral row passes:
+// One kernel's growth terms at a pixel pair:
 // bell(u) = exp(-(u - mu)^2 / (2 sigma^2)) = 2^-((u*sc - mu*sc)^2) with
 // sc = sqrt(log2(e) / 2) / sigma, and the term h * (2 bell - 1) (growth mode
 // 0) or h * bell (mode 1) as g1 * bell + g0 -- in packed FP32x2 pairs (one
@@ -107,6 +103,12 @@ struct GrowthPair {
     __device__ __forceinline__ float2 term(float2 u, float2 shift) const {
         return bells(make_float2((u.x - (mu + shift.x)) * sc, (u.y - (mu + shift.y)) * sc));
     }
+    // The same, its difference u - mu taken first (exact near mu): the direct
+    // paths' potentials carry less rounding than the transforms', and u * sc -
+    // mu * sc would add that of mu * sc.
+    __device__ __forceinline__ float2 term_near(float2 u, float2 shift) const {
+        return bells(__fmul2_rn(__fadd2_rn(u, make_float2(-(mu + shift.x), -(mu + shift.y))), SC));
+    }
     // d: (u - mu) * sc for both pixels.
     __device__ __forceinline__ float2 bells(float2 d) const {
         const float2 q = __fmul2_rn(d, d);
@@ -117,31 +119,22 @@ struct GrowthPair {
 
 __device__ __forceinline__ float bell_fast(float u, float mu, float inv_sigma) {
     const float t = (u - mu) * inv_sigma;
-    float r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(-0.72134752044448170368f * t * t));
-    return r;
+    return ex2_fast(-0.72134752044448170368f * t * t);
 }
-
-// Running growth sums over kernels in the reference's order
-// (Lenia.metal:188-195): sum_k h_k*bell_k and sum_k h_k*(2*bell_k - 1).
-struct GrowthAcc {
-    float weighted = 0.0f;
-    float std_sum = 0.0f;
-    __device__ __forceinline__ void add(float h, float b) {
-        weighted += h * b;
-        std_sum += h * (2.0f * b - 1.0f);
-    }
-};
 
 // Euler step (Lenia.metal:197-209, identical to leniaStep's for one kernel of
-// weight 1).
-__device__ __forceinline__ float growth_euler(const StepParams& p, float A, float weighted, float std_sum) {
-    if (p.growth_mode == 1u) {
-        const float target = (p.sum_weights > 1e-6f) ? (weighted / p.sum_weights) : A;
-        return A + p.dt * (target - A);
+// weight 1); s: the mode's growth sum, sum_k h_k * bell_k (asymptotic) or
+// sum_k h_k * (2 bell_k - 1), in kernel order (Lenia.metal:188-195). The
+// division by sum_k h_k is a product with its reciprocal, taken once.
+struct EulerStep {
+    float dt, inv_sum;
+    bool asym, weighted;
+    __device__ __forceinline__ explicit EulerStep(const StepParams& p)
+        : dt(p.dt), inv_sum(1.0f / p.sum_weights), asym(p.growth_mode == 1u), weighted(p.sum_weights > 1e-6f) {}
+    __device__ __forceinline__ float operator()(float A, float s) const {
+        return asym ? A + dt * ((weighted ? s * inv_sum : A) - A) : A + dt * s;
     }
-    return A + p.dt * std_sum;
-}
+};
 
 // Noise stir, blob injection and clip (Lenia.metal:210-231) of the N pixels
 // (gx, gy) .. (gx + N - 1, gy).
@@ -206,7 +199,8 @@ __device__ __forceinline__ void noise_inject_clip(const StepParams& p, const Gro
 // gy); s: the mode's growth sums.
 static __device__ __noinline__ float2 growth_finish_pair(const StepParams& p, const GrowthExtras& ex, float2 A,
                                                          float2 s, uint32_t gx, uint32_t gy) {
-    float v[2] = {growth_euler(p, A.x, s.x, s.x), growth_euler(p, A.y, s.y, s.y)};
+    const EulerStep euler(p);
+    float v[2] = {euler(A.x, s.x), euler(A.y, s.y)};
     noise_inject_clip(p, ex, v, gx, gy);
     return make_float2(v[0], v[1]);
 }

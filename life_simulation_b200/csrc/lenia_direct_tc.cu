@@ -1,0 +1,652 @@
+// life_simulation_b200/csrc/lenia_direct_tc.cu -- the direct toroidal
+// convolution as a banded GEMM on the tensor cores (tcgen05.mma kind::i8,
+// exact 32-bit integer accumulators in tensor memory), fused with the growth
+// epilogue: the same update as lenia_direct.cu (the work of leniaStep,
+// Shaders/Field/Lenia.metal:63-128, for up to 4 kernel tables).
+//
+// Arithmetic. A field value a in [0, 2) is the 24-bit fixed-point number
+// A = rint(a 2^23) = a0 2^16 + a1 2^8 + a2 (unsigned bytes), a weight w the
+// number rint(w 2^e) = w0 2^16 + w1 2^8 + w2 (signed bytes; e the largest
+// exponent that keeps the table in range). The products of byte i and byte j
+// go to the integer sum of level i + j; levels 0 to 3 (all but the last of the
+// nine products) are summed exactly -- 3 * 4225 taps * 255 * 128 < 2^31 -- and
+// combined in FP32 once: U = L0 2^(9-e) + (L1 + L2 / 2^8 + L3 / 2^16) 2^(1-e).
+// What is dropped is 2^-32 of a tap's share, so the sum's error is the
+// rounding of that last combination, where the FP32 form rounds once per tap;
+// and an integer sum is the same in any order. A tile whose halo holds a value outside [0, 2)
+// (an uploaded field may: infinities, NaN, negative values) takes the FP32
+// loop below, tap by tap in the order of lenia_direct.cu.
+//
+// The GEMM. A CTA owns 128 rows x 32 columns of output. Kernel row dy over a
+// chunk of 32 input columns is D[128 x 32] += X[128 x 32] T[32 x 32]: X is the
+// halo tile's rows dy .. dy + 127 (the accumulator's lanes are the output
+// rows), T the Toeplitz block T[k][n] = w(dy, base + k - n) of the chunk that
+// starts `base` columns beside the tile. A row of half width hw takes 1 + 2 Q
+// / 32 chunks, Q = hw rounded up to 16, so the disc's corners cost less. The
+// rows' shift by dy is 16 bytes in X's start address: both operands lie in
+// shared memory in 16-byte rows (K-major core matrices without swizzle, rows
+// evenly 16 bytes apart), so one staged tile serves every dy.
+//
+// What bounds it: the operands' shared-memory reads. A product of N columns
+// takes max(46, 32 + N / 4) cycles (measured, N <= 128: 4 KB of X and 32 N
+// bytes of T at 128 bytes a cycle, against N / 2 cycles of math), so small N
+// is lost; the levels of a chunk are side by side in D and T's byte planes in
+// [w0 | w1 | w2] rows, which makes the eight byte products three: X0 against
+// all of T (N = 96) into levels 0..2, X1 likewise into levels 1..3, X2 against
+// [w0 | w1] (N = 64) into levels 2 and 3: 161 cycles a chunk, where eight
+// products of N = 32 took 366. Wider tiles read X less often but clip T's
+// window, and came out behind. The T blocks (3 KB a chunk) come through a ring of bulk copies from
+// L2, requested by one warp and multiplied by another, whose loop is uniform
+// over the warp.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cmath>
+#include <cstddef>
+#include <cstdint>
+#include <vector>
+
+#include "fft_fast_common.cuh"
+#include "lenia_device.cuh"
+#include "lenia_kernels.h"
+
+namespace lenia {
+namespace {
+
+constexpr int kRows = 128;             // output rows of a tile (accumulator lanes)
+constexpr int kTX = 32;                // output columns of a tile
+constexpr int kPart = kTX / 2;         // output columns per epilogue thread
+// Warps: 0..7 epilogue (tensor-memory lane quadrant warp % 4, half of the
+// columns warp / 4), 8..15 stage the halo tiles, 16 and 17 issue the products
+// (a product is issued when the one before it in its warp has been read, so
+// one warp's waits leave the tensor cores idle; two warps on alternate T
+// blocks, each with its own accumulator, fill each other's), 18 requests the
+// T blocks.
+constexpr int kEpiWarps = 8, kStageWarps = 8, kMmaWarp = 16, kMmaWarps = 2, kLoadWarp = 18;
+constexpr int kThreads = 32 * 19;
+constexpr int kStages = 6;             // T blocks in flight
+constexpr uint32_t kCols = 512;        // tensor-memory columns: per buffer and issuing warp 128 (four levels)
+constexpr uint32_t kChunk = 96u * 32u; // bytes of one chunk's T: 96 rows of 32 k
+constexpr uint32_t kPolls = 1u << 20;  // polls of a barrier before a CTA gives up (about a second)
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) {
+    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+// Matrix descriptor (sm_100 format, no swizzle). Low word: start address and
+// leading byte offset (between the two 16-byte halves of K = 32), high word:
+// stride byte offset 128 (between groups of eight rows), all >> 4, and
+// descriptor version 1.
+__device__ __forceinline__ uint32_t desc_lo(uint32_t addr, uint32_t lbo) { return (addr >> 4) | ((lbo >> 4) << 16); }
+constexpr uint32_t kDescHi = (128u >> 4) | (1u << 14);
+// kind::i8, S32 accumulator (2), A unsigned bytes (0), B signed bytes (1),
+// both K-major, M = 128 (>> 4), N (>> 3).
+constexpr uint32_t idesc(uint32_t n) {
+    return (2u << 4) | (0u << 7) | (1u << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24);
+}
+
+// Issued by the one lane whose `lead` is set, in a converged warp: a
+// predicate on the instruction, not a branch around it, so that the loop
+// that computes the descriptors stays uniform and keeps them in uniform
+// registers (in a one-lane branch they cost 20 to 60 cycles a product). a, b:
+// low words of the operands' descriptors (their high words are constant).
+__device__ __forceinline__ void mma_i8(uint32_t d, uint32_t a, uint32_t b, uint32_t id, uint32_t acc, uint32_t lead) {
+    asm volatile(
+        "{\n .reg .pred p, q;\n .reg .b64 x, y;\n setp.ne.b32 p, %5, 0;\n setp.ne.b32 q, %6, 0;\n"
+        " mov.b64 x, {%1, %4};\n mov.b64 y, {%2, %4};\n"
+        " @q tcgen05.mma.cta_group::1.kind::i8 [%0], x, y, %3, p;\n}\n" ::"r"(d),
+        "r"(a), "r"(b), "r"(id), "r"(kDescHi), "r"(acc), "r"(lead)
+        : "memory");
+}
+__device__ __forceinline__ void commit(uint64_t* bar, uint32_t lead) {
+    asm volatile(
+        "{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n"
+        " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(smem_u32(bar)),
+        "r"(lead)
+        : "memory");
+}
+// The products of one kernel row: NQ + 1 chunks from operand addresses a, b;
+// PLANE: bytes of a byte plane, STEP: bytes of two granules (a chunk's 32
+// columns).
+template <int NQ, uint32_t PLANE, uint32_t STEP>
+__device__ __forceinline__ void mma_row(uint32_t tmem, uint32_t a, uint32_t b, uint32_t acc, uint32_t lead) {
+#pragma unroll
+    for (int c = 0; c <= NQ; ++c) {
+        const uint32_t ac = a + uint32_t(c) * (STEP / 16), bc = b + uint32_t(c) * (kChunk / 16);
+        mma_i8(tmem, ac, bc, idesc(96), c > 0 ? 1u : acc, lead);
+        mma_i8(tmem + kTX, ac + PLANE / 16, bc, idesc(96), 1, lead);
+        mma_i8(tmem + 2 * kTX, ac + 2 * (PLANE / 16), bc, idesc(64), 1, lead);
+    }
+}
+__device__ __forceinline__ void bar_init(uint64_t* bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ bool bar_try(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// Bounded, by a whole warp; false (for the whole warp) when the polls run out
+// or another warp's have (`stop`).
+__device__ __noinline__ bool bar_wait_slow(uint64_t* bar, uint32_t parity, volatile int* stop) {
+    for (uint32_t i = 0; i < kPolls; ++i) {
+        if (bar_try(bar, parity)) return true;
+        if ((i & 255u) == 255u && *stop) return false;
+    }
+    *stop = 1;
+    return false;
+}
+__device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity, volatile int* stop) {
+    bool ok = bar_try(bar, parity);
+    if (!__all_sync(0xffffffffu, ok)) ok = bar_wait_slow(bar, parity, stop);
+    return __all_sync(0xffffffffu, ok);
+}
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(bytes)
+                 : "memory");
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
+                     smem_u32(dst)),
+                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+}
+__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
+__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
+
+// 8 consecutive accumulator columns of this warp's lane quadrant (not
+// waited for).
+__device__ __forceinline__ void tmem_ld8(uint32_t addr, int32_t (&v)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(addr));
+}
+__device__ __forceinline__ void tmem_zero8(uint32_t addr) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1};\n" ::"r"(addr), "r"(0) : "memory");
+}
+
+__device__ __forceinline__ int wrap(int v, int n) {
+    if (v >= 0 && v < n) return v;
+    v %= n;
+    return v < 0 ? v + n : v;
+}
+
+// One output of the FP32 form (values the byte form cannot hold): taps in
+// the order of direct_tile.
+__device__ __noinline__ float direct_point(const float* __restrict__ src, const float* __restrict__ weights,
+                                           const uint32_t* __restrict__ spans, const DirectGeometry& g, int W, int H,
+                                           int k, int x, int y) {
+    float acc = 0.0f;
+    for (int dyi = 0; dyi < g.ksize; ++dyi) {
+        const uint32_t sp = spans[k * g.ksize + dyi];
+        const int start = int(sp & 0xFFFFu) - 128, count = int(sp >> 16);
+        const float* row = src + size_t(wrap(y + dyi - g.r, H)) * W;
+        const float* w = weights + size_t(k * g.ksize + dyi) * g.wp + g.xp;
+        for (int d = start; d < start + 8 * count; ++d) acc = fmaf(w[d], row[wrap(x + d, W)], acc);
+    }
+    return acc;
+}
+
+// Barriers and flags of a CTA.
+struct TcShared {
+    uint64_t t_full[kStages], t_empty[kStages];  // T blocks
+    uint64_t a_full[2], a_empty[2];              // staged halo tiles
+    uint64_t d_full[2], d_empty[2];              // accumulators
+    uint64_t drain[kMmaWarps];                              // products in flight when a wait ran out
+    int bad[4];     // tile count + 1 of the last tile of slot (count % 4) with a value outside the byte form
+    int stop;       // a wait ran out
+    uint32_t tmem;  // tensor-memory address
+    GrowthExtras ex;
+};
+
+// P: halo columns each side (16 for r <= 16, else 32); the staged planes have
+// 128 + 2 P rows, of which 128 + 2 r are read. One CTA per SM loops
+// over tiles; staging, products and epilogue of successive tiles overlap (two
+// staged tiles, two accumulators).
+template <int P>
+__global__ void __launch_bounds__(kThreads, 1)
+    direct_tc_kernel(const float* __restrict__ src, float* __restrict__ dst, const __grid_constant__ DirectTcPlan plan,
+                     const float* __restrict__ weights, const uint32_t* __restrict__ spans,
+                     const __grid_constant__ DirectGeometry g, const __grid_constant__ StepParams p, int nk,
+                     int tiles_x, int tiles, int* err) {
+    extern __shared__ __align__(128) unsigned char sm[];
+    __shared__ TcShared sh;
+    constexpr int RA = kRows + 2 * P, NG = (kTX + 2 * P) / 16;      // staged rows, 16-column granules
+    constexpr uint32_t kPlane = uint32_t(RA) * 16u * uint32_t(NG);  // bytes of one staged byte plane
+    constexpr uint32_t kStage = kChunk * uint32_t(1 + P / 16);
+    const int tid = int(threadIdx.x), warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const int W = int(p.width), H = int(p.height);
+    unsigned char* ring = sm + 6u * kPlane;
+
+    if (tid == 0) {
+        sh.stop = 0;
+        for (int i = 0; i < kStages; ++i) {
+            bar_init(&sh.t_full[i], 1);
+            bar_init(&sh.t_empty[i], 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            bar_init(&sh.a_full[i], kStageWarps);
+            bar_init(&sh.a_empty[i], kMmaWarps);
+            bar_init(&sh.d_full[i], kMmaWarps);
+            bar_init(&sh.d_empty[i], kEpiWarps);
+        }
+        for (int i = 0; i < kMmaWarps; ++i) bar_init(&sh.drain[i], 1);
+        for (int i = 0; i < 4; ++i) sh.bad[i] = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    if (warp == kMmaWarp) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&sh.tmem)),
+                     "r"(kCols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
+    growth_extras_init(sh.ex, p);
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, sh.tmem, 0);
+    // Level 3 starts at zero (the first product of a kernel sets levels 0 to
+    // 2); from then on the epilogue clears it as it reads it.
+    if (warp < kEpiWarps) {
+        const uint32_t at = tmem + (uint32_t(32 * (warp & 3)) << 16) + uint32_t(3 * kTX + kPart * (warp >> 2));
+#pragma unroll
+        for (int c = 0; c < kPart; c += 8)
+#pragma unroll
+            for (uint32_t d = 0; d < kCols; d += 128) tmem_zero8(at + d + uint32_t(c));
+        asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+        fence_before();
+    }
+    __syncthreads();
+
+    if (warp >= kEpiWarps && warp < kEpiWarps + kStageWarps) {
+        // ---- Stage the halo tiles as three byte planes, [16-column granule]
+        // [row][16 bytes]: a warp access covers eight rows of a granule, four
+        // lanes a row (64 bytes loaded; the 4-byte stores fill 128 contiguous
+        // bytes), five or six accesses in flight.
+        fastfft::grid_dependency_wait();
+        constexpr int kGroups = RA / 8, kItems = kGroups * NG, kFlight = P == 16 ? 5 : 6;
+        static_assert(kItems % (kFlight * kStageWarps) == 0, "whole batches of accesses");
+        const int q = 4 * (lane & 3), rl = lane >> 2;
+        uint32_t ai = 0;
+        for (int tile = int(blockIdx.x); tile < tiles; tile += int(gridDim.x), ++ai) {
+            const uint32_t buf = ai & 1u;
+            if (ai >= 2 && !bar_wait(&sh.a_empty[buf], ((ai >> 1) - 1u) & 1u, &sh.stop)) break;
+            const int ty = tile / tiles_x, x0 = (tile - ty * tiles_x) * kTX, y0 = ty * kRows;
+            const bool inside = W % 4 == 0 && x0 >= P && x0 + kTX + P <= W;
+            unsigned char* planes = sm + buf * 3u * kPlane;
+            bool bad = false;
+#pragma unroll 1
+            for (int i0 = warp - kEpiWarps; i0 < kItems; i0 += kFlight * kStageWarps) {
+                float4 a[kFlight];
+#pragma unroll
+                for (int f = 0; f < kFlight; ++f) {
+                    const int i = i0 + f * kStageWarps, gran = i / kGroups, row = (i - gran * kGroups) * 8 + rl;
+                    const float* line = src + size_t(wrap(y0 - g.r + row, H)) * W;
+                    const int x = x0 - P + 16 * gran + q;
+                    if (inside) {
+                        a[f] = __ldg(reinterpret_cast<const float4*>(line + x));
+                    } else {
+                        a[f].x = __ldg(line + wrap(x, W));
+                        a[f].y = __ldg(line + wrap(x + 1, W));
+                        a[f].z = __ldg(line + wrap(x + 2, W));
+                        a[f].w = __ldg(line + wrap(x + 3, W));
+                    }
+                }
+#pragma unroll
+                for (int f = 0; f < kFlight; ++f) {
+                    const int i = i0 + f * kStageWarps, gran = i / kGroups, row = (i - gran * kGroups) * 8 + rl;
+                    // 0 <= a < 2 exactly when the sign and the top exponent bit are
+                    // clear (-0 takes the FP32 form as well).
+                    bad = bad || (((__float_as_uint(a[f].x) | __float_as_uint(a[f].y)) |
+                                   (__float_as_uint(a[f].z) | __float_as_uint(a[f].w))) &
+                                  0xC0000000u) != 0u;
+                    const uint32_t v0 = __float2uint_rn(a[f].x * 8388608.0f), v1 = __float2uint_rn(a[f].y * 8388608.0f);
+                    const uint32_t v2 = __float2uint_rn(a[f].z * 8388608.0f), v3 = __float2uint_rn(a[f].w * 8388608.0f);
+                    const uint32_t l01 = __byte_perm(v0, v1, 0x5140), l23 = __byte_perm(v2, v3, 0x5140);
+                    const uint32_t h01 = __byte_perm(v0, v1, 0x7362), h23 = __byte_perm(v2, v3, 0x7362);
+                    unsigned char* o = planes + (gran * RA + row) * 16 + q;
+                    *reinterpret_cast<uint32_t*>(o) = __byte_perm(h01, h23, 0x5410);
+                    *reinterpret_cast<uint32_t*>(o + kPlane) = __byte_perm(l01, l23, 0x7632);
+                    *reinterpret_cast<uint32_t*>(o + 2 * kPlane) = __byte_perm(l01, l23, 0x5410);
+                }
+            }
+            if (bad) *reinterpret_cast<volatile int*>(&sh.bad[ai & 3u]) = int(ai) + 1;
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+            __syncwarp();
+            if (lane == 0) bar_arrive(&sh.a_full[buf]);
+        }
+        fastfft::allow_dependents();
+    } else if (warp == kLoadWarp) {
+        // ---- T blocks (tables: they do not depend on the step before).
+        uint32_t ti = 0;
+        for (int tile = int(blockIdx.x); tile < tiles; tile += int(gridDim.x)) {
+            uint32_t offset = 0;
+#pragma unroll 1
+            for (int r = 0; r < plan.first[nk]; ++r, ++ti) {
+                const uint32_t st = ti % kStages, bytes = kChunk * (1u + (uint32_t(plan.rows[r]) >> 14));
+                if (ti >= kStages && !bar_wait(&sh.t_empty[st], (ti / kStages - 1u) & 1u, &sh.stop)) break;
+                if (lane == 0) bulk_load(ring + st * kStage, plan.blocks + offset, bytes, &sh.t_full[st]);
+                offset += bytes;
+            }
+            if (*reinterpret_cast<volatile int*>(&sh.stop)) break;
+        }
+        // After a wait ran out: the copies in flight get one more bounded wait.
+        if (*reinterpret_cast<volatile int*>(&sh.stop)) {
+            int never = 0;
+            for (uint32_t i = ti > kStages ? ti - kStages : 0; i < ti; ++i)
+                bar_wait_slow(&sh.t_full[i % kStages], (i / kStages) & 1u, &never);
+        }
+    } else if (warp >= kMmaWarp && warp < kMmaWarp + kMmaWarps) {
+        // ---- Products of every second T block.
+        const int m = warp - kMmaWarp;
+        uint32_t lead;
+        asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(lead));
+        const uint32_t b_base = desc_lo(smem_u32(ring), kChunk / 2);
+        uint32_t ai = 0, di = 0, st = 0, ph = 0;  // ring stage and its phase
+        bool ok = true;
+        for (int tile = int(blockIdx.x); tile < tiles && ok; tile += int(gridDim.x), ++ai) {
+            const uint32_t buf = ai & 1u;
+            const uint32_t a_base = desc_lo(smem_u32(sm) + buf * 3u * kPlane, RA * 16u) + uint32_t((P / 16) * RA);
+            ok = bar_wait(&sh.a_full[buf], (ai >> 1) & 1u, &sh.stop);
+#pragma unroll 1
+            for (int k = 0; k < nk && ok; ++k, ++di) {
+                const uint32_t db = di & 1u, d = tmem + db * 256u + uint32_t(m) * 128u;
+                if (di >= 2) ok = bar_wait(&sh.d_empty[db], ((di >> 1) - 1u) & 1u, &sh.stop);
+                fence_after();
+                uint32_t acc = 0;  // the first product of N = 96 sets the accumulator
+                const int r0 = plan.first[k], r1 = plan.first[k + 1];
+#pragma unroll 1
+                for (int r = r0; r < r1 && ok; ++r) {
+                    if (((r - r0) & 1) == m) {
+                        const uint32_t row = plan.rows[r], nq = row >> 14;
+                        const uint32_t a = a_base - nq * uint32_t(RA), b = b_base + st * (kStage / 16);
+                        const uint32_t dy0 = row & 127u, dy1 = (row >> 7) & 127u;
+                        ok = bar_wait(&sh.t_full[st], ph, &sh.stop);
+                        if (!ok) break;
+                        if (P == 32 && nq == 2) {
+                            mma_row<2, kPlane, 32u * RA>(d, a + dy0, b, acc, lead);
+                            if (dy1 != dy0) mma_row<2, kPlane, 32u * RA>(d, a + dy1, b, 1u, lead);
+                        } else if (nq == 1) {
+                            mma_row<1, kPlane, 32u * RA>(d, a + dy0, b, acc, lead);
+                            if (dy1 != dy0) mma_row<1, kPlane, 32u * RA>(d, a + dy1, b, 1u, lead);
+                        } else {
+                            mma_row<0, kPlane, 32u * RA>(d, a + dy0, b, acc, lead);
+                            if (dy1 != dy0) mma_row<0, kPlane, 32u * RA>(d, a + dy1, b, 1u, lead);
+                        }
+                        acc = 1;
+                        commit(&sh.t_empty[st], lead);
+                    }
+                    if (++st == kStages) st = 0, ph ^= 1u;
+                }
+                if (ok) commit(&sh.d_full[db], lead);
+            }
+            if (ok) commit(&sh.a_empty[buf], lead);
+        }
+    } else {
+        // ---- Epilogue: growth sums of row y0 + 32 (warp % 4) + lane, columns
+        // x0 + kPart (warp / 4) .. + kPart - 1, over the kernels; then A'.
+        fastfft::grid_dependency_wait();
+        const int quad = warp & 3, half = warp >> 2;
+        const uint32_t mine = tmem + (uint32_t(32 * quad) << 16) + uint32_t(kPart * half);
+        const EulerStep euler(p);
+        const bool jitter = p.mu_jitter > 0.0f;
+        // Selects instead of a dynamic index into the parameter block (which
+        // would spill it to local memory).
+        const auto pick = [](const float(&a)[kMaxKernels], int k) {
+            return k == 0 ? a[0] : k == 1 ? a[1] : k == 2 ? a[2] : a[3];
+        };
+        uint32_t ai = 0, di = 0;
+        bool ok = true;
+        for (int tile = int(blockIdx.x); tile < tiles && ok; tile += int(gridDim.x), ++ai) {
+            const int ty = tile / tiles_x, gx0 = (tile - ty * tiles_x) * kTX + kPart * half;
+            const int gy = ty * kRows + 32 * quad + lane;
+            // This thread's values of A, requested before the products are waited
+            // for (rows past the field read its last one).
+            const float* arow = src + size_t(min(gy, H - 1)) * W;
+            float4 av[kPart / 4];
+            const bool whole = W % 4 == 0 && gx0 + kPart <= W;
+#pragma unroll
+            for (int c = 0; c < kPart / 4; ++c) {
+                if (whole) {
+                    av[c] = __ldg(reinterpret_cast<const float4*>(arow + gx0) + c);
+                } else {
+                    const int x = gx0 + 4 * c;
+                    av[c].x = x < W ? __ldg(arow + x) : 0.0f;
+                    av[c].y = x + 1 < W ? __ldg(arow + x + 1) : 0.0f;
+                    av[c].z = x + 2 < W ? __ldg(arow + x + 2) : 0.0f;
+                    av[c].w = x + 3 < W ? __ldg(arow + x + 3) : 0.0f;
+                }
+            }
+            float2 sum[kPart / 2];  // growth sums of pixel pairs
+#pragma unroll 1
+            for (int k = 0; k < nk; ++k, ++di) {
+                const uint32_t db = di & 1u;
+                if (!(ok = bar_wait(&sh.d_full[db], (di >> 1) & 1u, &sh.stop))) break;
+                fence_after();
+                const bool bytes = *reinterpret_cast<volatile int*>(&sh.bad[ai & 3u]) != int(ai) + 1;
+                const float scale = pick(plan.scale, k);
+                const float s0 = scale * 512.0f, s1 = scale * 2.0f;
+                const GrowthPair gp(pick(p.mu, k), 1.0f / pick(p.sigma, k), pick(p.weight, k), euler.asym);
+                const bool two = plan.first[k + 1] - plan.first[k] > 1;  // T blocks for the second issuing warp
+#pragma unroll
+                for (int c = 0; c < kPart; c += 8) {
+                    float u[8];
+                    int32_t l0[8], l1[8], l2[8], l3[8], m0[8] = {}, m1[8] = {}, m2[8] = {}, m3[8] = {};
+                    const uint32_t d = mine + db * 256u + uint32_t(c);
+                    tmem_ld8(d, l0);
+                    tmem_ld8(d + kTX, l1);
+                    tmem_ld8(d + 2 * kTX, l2);
+                    tmem_ld8(d + 3 * kTX, l3);
+                    if (two) {
+                        tmem_ld8(d + 128, m0);
+                        tmem_ld8(d + 128 + kTX, m1);
+                        tmem_ld8(d + 128 + 2 * kTX, m2);
+                        tmem_ld8(d + 128 + 3 * kTX, m3);
+                    }
+                    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+                    tmem_zero8(d + 3 * kTX);
+                    tmem_zero8(d + 128 + 3 * kTX);
+                    // Levels 2 and 3 join level 1 as integers (rounded at 2^-31 of the sum).
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const int32_t v2 = l2[j] + m2[j] + ((l3[j] + m3[j] + 128) >> 8);
+                        const int32_t v1 = l1[j] + m1[j] + ((v2 + 128) >> 8);
+                        u[j] = fmaf(float(l0[j] + m0[j]), s0, float(v1) * s1);
+                    }
+                    if (!bytes) {
+#pragma unroll 1
+                        for (int j = 0; j < 8; ++j) {
+                            const float v = gy < H && gx0 + c + j < W
+                                                ? direct_point(src, weights, spans, g, W, H, k, gx0 + c + j, gy)
+                                                : 0.0f;
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) u[i] = i == j ? v : u[i];
+                        }
+                    }
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float2 uu = make_float2(u[2 * j], u[2 * j + 1]);
+                        const float2 t =
+                            gp.term_near(uu, jitter ? mu_jitter_pair(p, sh.ex, uint32_t(gx0 + c + 2 * j), uint32_t(gy))
+                                                    : make_float2(0.0f, 0.0f));
+                        float2& to = sum[c / 2 + j];
+                        to = k == 0 ? t : __fadd2_rn(to, t);
+                    }
+                }
+                asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+                fence_before();
+                __syncwarp();
+                if (lane == 0) bar_arrive(&sh.d_empty[db]);
+            }
+            if (!ok) break;  // its tile is left unwritten
+            if (gy >= H) continue;
+            float* orow = dst + size_t(gy) * W;
+#pragma unroll
+            for (int c = 0; c < kPart; c += 8) {
+                const int gx = gx0 + c;
+                const float4 a = av[c / 4], b = av[c / 4 + 1];
+                float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    v[2 * j] = euler(v[2 * j], sum[c / 2 + j].x);
+                    v[2 * j + 1] = euler(v[2 * j + 1], sum[c / 2 + j].y);
+                }
+                noise_inject_clip(p, sh.ex, v, uint32_t(gx), uint32_t(gy));
+                if (whole) {
+                    float4* o = reinterpret_cast<float4*>(orow + gx);
+                    o[0] = make_float4(v[0], v[1], v[2], v[3]);
+                    o[1] = make_float4(v[4], v[5], v[6], v[7]);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        if (gx + j < W) orow[gx + j] = v[j];
+                }
+            }
+        }
+    }
+    fence_before();
+    __syncthreads();
+    if (*reinterpret_cast<volatile int*>(&sh.stop)) {
+        // A wait ran out: products still in flight get one more bounded wait
+        // before their accumulators are freed.
+        if (warp >= kMmaWarp && warp < kMmaWarp + kMmaWarps) {
+            int never = 0;
+            fence_after();
+            commit(&sh.drain[warp - kMmaWarp], lane == 0 ? 1u : 0u);
+            bar_wait_slow(&sh.drain[warp - kMmaWarp], 0, &never);
+        }
+        __syncthreads();
+    }
+    if (warp == kMmaWarp)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kCols));
+    if (tid == 0 && *reinterpret_cast<volatile int*>(&sh.stop) && err) atomicAdd(err, 1);
+}
+
+template <int P>
+cudaError_t launch_t(int nk, const float* src, float* dst, const DirectTcPlan& plan, const float* weights,
+                     const uint32_t* spans, const DirectGeometry& g, const StepParams& p, int* err, cudaStream_t s) {
+    auto fn = direct_tc_kernel<P>;
+    constexpr size_t smem = 6 * size_t(kRows + 2 * P) * (kTX + 2 * P) + size_t(kStages) * kChunk * (1 + P / 16);
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    if (e != cudaSuccess) return e;
+    const int tx = int((p.width + kTX - 1) / kTX), tiles = tx * int((p.height + kRows - 1) / kRows);
+    return fastfft::launch_chained(fn, dim3(unsigned(std::min(tiles, fastfft::sms()))), kThreads, smem, s, src, dst,
+                                   plan, weights, spans, g, p, nk, tx, tiles, err);
+}
+
+}  // namespace
+
+// The T blocks of the kernel tables ((2r + 1)^2 weights each) in the order of
+// the plan's rows: per kernel row with a nonzero weight and per chunk, two
+// halves of k x 96 rows (byte plane j, output n) x 16 values of k.
+bool direct_tc_tables(const std::vector<std::vector<float>>& luts, int r, DirectTcTables& out) {
+    out = DirectTcTables();
+    if (r < 0 || r > kMaxRadius || luts.empty() || luts.size() > size_t(kMaxKernels)) return false;
+    const int ks = 2 * r + 1;
+    int rows = 0;
+    for (size_t k = 0; k < luts.size(); ++k) {
+        const std::vector<float>& lut = luts[k];
+        if (lut.size() != size_t(ks) * ks) return false;
+        float top = 0.0f;
+        for (float w : lut) {
+            if (!std::isfinite(w)) return false;
+            top = std::max(top, std::fabs(w));
+        }
+        // The largest e with top * 2^e within three signed bytes.
+        if (!(top > 0.0f)) return false;
+        int e = 0;
+        std::frexp(8355711.0 / double(top), &e);
+        e -= 1;  // 2^e <= 8355711 / top < 2^(e + 1)
+        if (e > 100) return false;
+        out.plan.scale[k] = float(std::ldexp(1.0, -e));
+        out.plan.first[k] = rows;
+        double carry = 0.0;
+        int taps = 0;
+        for (float w : lut) taps += w != 0.0f;
+        out.min_taps = k == 0 ? taps : std::min(out.min_taps, taps);
+        const auto row_at = [&](int dyi) { return lut.begin() + std::ptrdiff_t(dyi) * ks; };
+        for (int dyi = 0; dyi < ks; ++dyi) {
+            // Rows dy and -dy of a radial kernel are the same weights and share
+            // one T block (the pair runs at the first of them).
+            const int twin = 2 * r - dyi;
+            const bool same = std::equal(row_at(dyi), row_at(dyi) + ks, row_at(twin));
+            if (same && twin < dyi) continue;
+            int hw = -1;
+            std::vector<int32_t> wi(size_t(ks), 0);
+            for (int dx = -r; dx <= r; ++dx) {
+                // Rounded with the error of the weights before it, so that the
+                // table's sum (1, or the scene's) is kept.
+                const double w = std::ldexp(double(lut[size_t(dyi) * ks + size_t(dx + r)]), e);
+                if (w == 0.0) continue;
+                const double x = std::min(std::max(w + carry, -8355711.0), 8355711.0);
+                const int32_t v = int32_t(std::llrint(x));
+                carry += w - double(v);
+                wi[size_t(dx + r)] = v;
+                if (v != 0) hw = std::max(hw, std::abs(dx));
+            }
+            if (hw < 0) continue;
+            const int nq = (hw + 15) / 16;
+            const size_t at = out.blocks.size();
+            out.blocks.resize(at + size_t(1 + nq) * kChunk, 0);
+            for (int c = 0; c <= nq; ++c)
+                for (int n = 0; n < kTX; ++n)
+                    for (int kk = 0; kk < 32; ++kk) {
+                        const int dx = 32 * c - 16 * nq + kk - n;
+                        if (dx < -hw || dx > hw) continue;
+                        const int32_t v = wi[size_t(dx + r)];
+                        // Signed bytes: v = d0 2^16 + d1 2^8 + d2, each in [-128, 127].
+                        const int32_t d2 = int32_t(int8_t(v & 0xFF)), v1 = (v - d2) / 256;
+                        const int32_t d1 = int32_t(int8_t(v1 & 0xFF)), d0 = (v1 - d1) / 256;
+                        const int32_t d[3] = {d0, d1, d2};
+                        for (int j = 0; j < 3; ++j)
+                            out.blocks[at + size_t(c) * kChunk + size_t(kk / 16) * (kChunk / 2) +
+                                       size_t(j * kTX + n) * 16 + size_t(kk % 16)] = uint8_t(int8_t(d[j]));
+                    }
+            out.chunks += (1 + nq) * (same && twin != dyi ? 2 : 1);
+            out.plan.rows[rows++] = uint16_t(dyi | ((same ? twin : dyi) << 7) | (nq << 14));
+        }
+    }
+    for (size_t k = luts.size(); k <= size_t(kMaxKernels); ++k) out.plan.first[k] = rows;
+    return true;
+}
+
+// Frame times in us as measured back to back on a B200 (148 SMs), one kernel:
+//                      R = 3        5        9        13       20       32
+//   128 x 128   FP32    7.1      9.1      9.1      11.2     13.3     21.7
+//               bytes   9.4     10.0     11.4      12.6     20.0     26.7
+//   512 x 512   FP32    9.1     11.2     15.3      19.4     29.7     62.4
+//               bytes   9.7     10.3     11.6      13.1     20.7     27.2
+//   1280 x 720  FP32   13.3     19.5     31.9      48.1     84.3    197.6
+//               bytes  13.4     14.2     15.8      18.4     30.2     44.1
+//   1920 x 1080 FP32   19.4     30.4     55.6      76.7    150.7    345.8
+//               bytes  21.1     22.8     27.1      32.3     47.4     74.8
+// (before the byte form the FP32 column was 205 us at 1280 x 720, R = 32 and 81
+// at 1920 x 1080, R = 13). Both sides are modelled from them: the byte form by
+// its fixed 8.5 us (launch, first tile's staging, last epilogue) and, per round
+// of tiles over the SMs, the larger of the products (87 ns a chunk) and the
+// staging and epilogue (3.4 us); the FP32 form by its 8-tap multiply-adds (3.7e-8
+// us each on fields that fill the SMs evenly, 4.8e-8 below) and 5e-6 us a
+// pixel. Kernels of few taps stay on the FP32 form, whose rounding grows with
+// the taps while the byte form's is fixed (they cross at R = 4, 49 taps).
+bool direct_tc_faster(const DirectTcTables& t, uint64_t fp32_taps, int w, int h, int sms) {
+    if (t.min_taps < 60) return false;
+    const double px = double(w) * h;
+    const int tiles = ((w + kTX - 1) / kTX) * ((h + kRows - 1) / kRows), rounds = (tiles + sms - 1) / std::max(1, sms);
+    const double bytes = 8.5 + rounds * std::max(0.087 * t.chunks, 3.4);
+    const double fp32 = 7.0 + px * (double(fp32_taps) * (px < 1.5e6 ? 4.8e-8 : 3.7e-8) + 5e-6);
+    return bytes < fp32;
+}
+
+cudaError_t launch_direct_tc(int nk, const float* src, float* dst, const DirectTcPlan& plan, const float* weights,
+                             const uint32_t* spans, const DirectGeometry& g, const StepParams& p, int* err,
+                             cudaStream_t s) {
+    if (nk < 1 || nk > kMaxKernels) return cudaErrorInvalidValue;
+    return g.r <= 16 ? launch_t<16>(nk, src, dst, plan, weights, spans, g, p, err, s)
+                     : launch_t<32>(nk, src, dst, plan, weights, spans, g, p, err, s);
+}
+
+}  // namespace lenia

@@ -188,24 +188,13 @@ __global__ void row_c2r_growth_kernel(FftGeometry g, const float2* __restrict__ 
             }
             __syncthreads();
             const float2* z = fft::run<true>(bb, ba, g.row, rows, tw);
-            const float mu = p.mu[kk], sigma = p.sigma[kk], h = p.weight[kk];
+            const GrowthPair gp(p.mu[kk], 1.0f / p.sigma[kk], p.weight[kk], asym);
             for (int q = threadIdx.x; q < M * rows; q += blockDim.x) {
                 const int r = q / M, n = q - r * M;
-                const float2 u = z[q];
-                const uint32_t gy = uint32_t(y0 + r);
-                float* ar = acc + r * W + 2 * n;
-                const float2 j = jitter ? mu_jitter_pair(p, ex, uint32_t(2 * n), gy) : make_float2(0.0f, 0.0f);
-                const float m0 = mu + j.x, m1 = mu + j.y;
-                const float bl0 = bell(u.x, m0, sigma), bl1 = bell(u.y, m1, sigma);
-                const float c0 = asym ? h * bl0 : h * (2.0f * bl0 - 1.0f);
-                const float c1 = asym ? h * bl1 : h * (2.0f * bl1 - 1.0f);
-                if (kk == 0) {
-                    ar[0] = c0;
-                    ar[1] = c1;
-                } else {
-                    ar[0] += c0;
-                    ar[1] += c1;
-                }
+                const float2 c = jitter ? gp.term(z[q], mu_jitter_pair(p, ex, uint32_t(2 * n), uint32_t(y0 + r)))
+                                        : gp.term(z[q]);
+                float2* ar = reinterpret_cast<float2*>(acc) + q;
+                *ar = kk == 0 ? c : __fadd2_rn(*ar, c);
             }
             __syncthreads();
         }

@@ -308,8 +308,7 @@ __global__ void __launch_bounds__(RowK<PI, RB, SPLIT>::T,
     // path reads them from the shared block out of line).
     const bool extras = p.noise_amount > 0.0f || p.inject_amount > 0.0f;
     if (extras || jitter) growth_extras_init(ex, p);  // visible after the first staged item's barrier
-    const float dt = p.dt, sum_w = p.sum_weights;
-    const bool sw_ok = sum_w > 1e-6f;
+    const EulerStep euler(p);
     // Item idx of a row group: the rows of U_idx for idx < nk, else of A.
     const auto stage = [&](float2* dst, int y, int idx) {
         if (y >= H) return;
@@ -420,12 +419,9 @@ __global__ void __launch_bounds__(RowK<PI, RB, SPLIT>::T,
                 }
                 // The common case (no noise, no injection) inline, its
                 // parameters in registers.
-                const auto finish = [&](float A, float s) {
-                    const float A2 = asym ? A + dt * ((sw_ok ? s / sum_w : A) - A) : A + dt * s;
-                    return fminf(fmaxf(A2, 0.0f), 1.0f);
-                };
                 const float2 r = extras ? growth_finish_pair(p, ex, a, acc[it][t], uint32_t(2 * n), uint32_t(gy))
-                                        : make_float2(finish(a.x, acc[it][t].x), finish(a.y, acc[it][t].y));
+                                        : make_float2(fminf(fmaxf(euler(a.x, acc[it][t].x), 0.0f), 1.0f),
+                                                      fminf(fmaxf(euler(a.y, acc[it][t].y), 0.0f), 1.0f));
                 *reinterpret_cast<float2*>(A_out + size_t(gy) * W + 2 * n) = r;
                 if constexpr (CM) palette_pair(sw.cm, r, sw.rgba + size_t(gy) * W + 2 * n);
                 za[it][t] = r;

@@ -67,6 +67,33 @@ cudaError_t launch_direct_step(int tile_cfg, int nk, const float* src, float* ds
 // Extra shared memory of a split direct launch (the groups' partial sums).
 size_t direct_split_smem_bytes(int split, int nk);
 
+// The direct step on the tensor cores (lenia_direct_tc.cu): weights as byte
+// planes of Toeplitz blocks, for each kernel row with a nonzero weight.
+struct DirectTcPlan {
+    const unsigned char* blocks = nullptr;  // device, 16-byte aligned
+    int first[kMaxKernels + 1] = {};        // rows of kernel k: [first[k], first[k + 1])
+    float scale[kMaxKernels] = {};          // 2^-e of kernel k's weights
+    // Kernel row | the row with the same weights on the other side << 7 | chunks - 1 << 14.
+    uint16_t rows[kMaxKernels * (2 * kMaxRadius + 1)] = {};
+};
+struct DirectTcTables {
+    std::vector<uint8_t> blocks;
+    DirectTcPlan plan;
+    int chunks = 0;    // chunks of 32 columns that a tile multiplies, all kernels
+    int min_taps = 0;  // nonzero weights of the smallest kernel
+};
+// Tables of nk (1..4) kernel tables of (2r + 1)^2 weights; false when they
+// have no byte form (a weight that is not finite, a kernel without weights).
+bool direct_tc_tables(const std::vector<std::vector<float>>& luts, int r, DirectTcTables& out);
+// Whether the tensor-core step is the one to run on a w x h field, against
+// launch_direct_step, which executes fp32_taps multiply-adds a pixel.
+bool direct_tc_faster(const DirectTcTables& t, uint64_t fp32_taps, int w, int h, int sms);
+// weights / spans / g: the FP32 tables (tiles whose values have no byte form
+// use them). err counts CTAs whose wait ran out.
+cudaError_t launch_direct_tc(int nk, const float* src, float* dst, const DirectTcPlan& plan, const float* weights,
+                             const uint32_t* spans, const DirectGeometry& g, const StepParams& p, int* err,
+                             cudaStream_t s);
+
 // -------------------------------------------------------------------- FFT
 constexpr int kMaxPasses = 8;
 

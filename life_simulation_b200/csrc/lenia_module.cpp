@@ -507,6 +507,9 @@ void LeniaModule::release() {
     direct_tma_ = DirectTma();
     rel(d_weights_);
     rel(d_spans_);
+    rel(d_tc_blocks_);
+    direct_tc_on_ = false;
+    direct_tc_ = DirectTcPlan();
     rel(d_org_);
     rel(d_S_);
     rel(d_U_);
@@ -804,6 +807,31 @@ int LeniaModule::buildDirectTables() {
         while (direct_split_ > 1 && direct_smem_bytes(direct_tile_, direct_nk_, dgeo_) +
                                             direct_split_smem_bytes(direct_split_, direct_nk_) > 220 * 1024)
             direct_split_ /= 2;
+    }
+    // The tensor-core step where it is the faster one (a rule on the size and
+    // radius). The variables that pick an FP32 kernel shape keep the FP32
+    // kernels; LENIA_DIRECT_ENGINE at setup forces either ("ffma", "tensor").
+    {
+        const char* eng = std::getenv("LENIA_DIRECT_ENGINE");
+        const std::string want = eng ? eng : "";
+        const bool shaped = std::getenv("LENIA_DIRECT_OX") || std::getenv("LENIA_DIRECT_OY") || std::getenv("LENIA_DIRECT_TMA");
+        uint64_t taps = 0;
+        for (uint32_t sp : spans) taps += 8u * (sp >> 16);
+        DirectTcTables t;
+        if (want != "ffma" && (want == "tensor" || !shaped) && direct_tc_tables(luts, r, t) &&
+            (want == "tensor" || direct_tc_faster(t, taps, int(w_), int(h_), sms))) {
+            if ((e = dev_alloc(&d_tc_blocks_, t.blocks.size(), device_bytes_)) != cudaSuccess ||
+                (e = dev_alloc(&d_tma_err_, 1, device_bytes_)) != cudaSuccess)
+                return cudaFail(e, "cudaMalloc direct tables");
+            cudaMemcpy(d_tc_blocks_, t.blocks.data(), t.blocks.size(), cudaMemcpyHostToDevice);
+            cudaMemset(d_tma_err_, 0, sizeof(int));
+            direct_tc_ = t.plan;
+            direct_tc_.blocks = d_tc_blocks_;
+            direct_tc_on_ = true;
+            direct_ox_ = 8;
+            direct_oy_ = 1;
+            return LENIA_OK;
+        }
     }
     // Outputs per thread on large tiles: 8 or 16 along x (64x32 tiles) times 1
     // or 2 rows (64x32 and 64x16 tiles, no split), whichever runs fastest here
@@ -1355,6 +1383,9 @@ int LeniaModule::stepImpl(const lenia_frame_params& fp, uint32_t substeps, cudaS
             spectrum_valid_ = true;
         } else {
             e = launch(LENIA_PHASE_DIRECT, s, [&] {
+                if (direct_tc_on_)
+                    return launch_direct_tc(direct_nk_, src, dst, direct_tc_, d_weights_, d_spans_, dgeo_, p, d_tma_err_,
+                                            s);
                 return launch_direct_step(direct_tile_, direct_nk_, src, dst, d_weights_, d_spans_, dgeo_, p, s,
                                           &direct_tma_, cur_, direct_split_, direct_ox_, direct_oy_);
             });

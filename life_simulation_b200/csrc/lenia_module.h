@@ -195,6 +195,10 @@ private:
     int* d_tma_err_ = nullptr;      // halo loads (direct) or MMA waits (tcgen05 column pass) that ran out
     float* d_weights_ = nullptr;
     uint32_t* d_spans_ = nullptr;
+    // The tensor-core form of the direct step (false: the FP32 kernels run).
+    bool direct_tc_on_ = false;
+    DirectTcPlan direct_tc_;
+    unsigned char* d_tc_blocks_ = nullptr;
     float* d_org_ = nullptr;
     float2* d_S_ = nullptr;
     float2* d_U_ = nullptr;
