@@ -20,6 +20,11 @@ constexpr int KB = kSpectralBlock;  // columns per block of the blocked layout
 
 constexpr int roundup32(int x) { return (x + 31) / 32 * 32; }
 
+// Blocks of a half spectrum of M columns (the last one padded when M is not
+// a whole number of blocks), and the columns a plane then holds.
+constexpr __host__ __device__ int blocks_of(int M) { return (M + KB - 1) / KB; }
+constexpr __host__ __device__ int padded_columns(int M) { return blocks_of(M) * KB; }
+
 // Smallest pitch >= n with 2*pitch = 8 (mod 32) (in float2): transforms of a
 // batch start 8 banks apart.
 constexpr int row_pitch(int n) {
@@ -135,6 +140,10 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
 }
+__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
+    const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
+}
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // Launch geometry of a column pass over B columns per CTA iteration (forward
@@ -166,12 +175,11 @@ template <class PI, int RB, int S = 1>
 struct RowK {
     using PF = typename Reverse<PI>::type;
     static constexpr int M = PI::n;
-    static_assert(M % KB == 0, "row length must be a whole number of blocks");
     static constexpr int RC = PI::last();
     static constexpr int NRC = M / RC;
     static constexpr int T = roundup32((RB * NRC + S - 1) / S);
     static constexpr int ITL = (RB * NRC + T - 1) / T;
-    static constexpr int PITCH = row_pitch(M);  // even: rows start 16-byte aligned
+    static constexpr int PITCH = row_pitch(padded_columns(M));  // even: rows start 16-byte aligned
     // Twiddle tables, then the buffers from an even float2 offset so the
     // 16-byte cp.async destinations are 16-byte aligned.
     static constexpr int TABLES = (M + 1) + PI::tw_size() + PF::tw_size();
@@ -191,7 +199,7 @@ struct RowK {
 // waits (cp_async_wait_all + barrier).
 template <int M, int RB, int T, int PITCH>
 __device__ __forceinline__ void stage_rows(float2* dst, const float2* __restrict__ plane, int H, int y0, int rows) {
-    for (int q = threadIdx.x; q < (M / KB) * RB * (KB / 2); q += T) {
+    for (int q = threadIdx.x; q < blocks_of(M) * RB * (KB / 2); q += T) {
         const int c2 = q % (KB / 2);
         const int b = (q / (KB / 2)) % RB;
         const int kb = q / ((KB / 2) * RB);
@@ -201,9 +209,17 @@ __device__ __forceinline__ void stage_rows(float2* dst, const float2* __restrict
 
 // Stages rows y0..y0+rows-1 of a row-major real field (W = 2M floats per
 // row) into shared rows of pitch PITCH, as M float2 pairs (x[2n], x[2n+1]):
-// 16-byte asynchronous copies. The caller waits.
+// 16-byte asynchronous copies, or 8-byte ones when M is odd (rows then start
+// 8 bytes off every other time). The caller waits.
 template <int M, int RB, int T, int PITCH>
 __device__ __forceinline__ void stage_field_rows(float2* dst, const float* __restrict__ field, int y0, int rows) {
+    if constexpr (M % 2 != 0) {
+        for (int q = threadIdx.x; q < RB * M; q += T) {
+            const int c = q % M, b = q / M;
+            if (b < rows) cp_async8(dst + b * PITCH + c, field + (size_t(y0 + b) * M + c) * 2);
+        }
+        return;
+    }
     for (int q = threadIdx.x; q < RB * (M / 2); q += T) {
         const int c = q % (M / 2), b = q / (M / 2);
         if (b < rows) cp_async16(dst + b * PITCH + 2 * c, field + (size_t(y0 + b) * M + 2 * c) * 2);
@@ -235,16 +251,20 @@ __device__ __forceinline__ float2 c2r_split(const float2* xr, const float2* twr,
 template <int M, int RB, int T, int PITCH>
 __device__ __forceinline__ void r2c_store_rows(const float2* Z, const float2* twr, float2* __restrict__ plane, int H,
                                                int y0, int rows) {
-    for (int q = threadIdx.x; q < (M / KB) * RB * (KB / 2); q += T) {
+    for (int q = threadIdx.x; q < blocks_of(M) * RB * (KB / 2); q += T) {
         const int c2 = q % (KB / 2);
         const int b = (q / (KB / 2)) % RB;
         const int kb = q / ((KB / 2) * RB);
-        if (b >= rows) continue;
+        if (b >= rows || (M % KB != 0 && kb * KB + 2 * c2 >= M)) continue;
         const float2* zr = Z + b * PITCH;
         float2 xv[2];
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             const int k = kb * KB + 2 * c2 + e;
+            if (M % 2 != 0 && k >= M) {  // the padding column beside an odd M's last
+                xv[e] = make_float2(0.0f, 0.0f);
+                continue;
+            }
             const float2 Zk = zr[k];
             if (k == 0) {
                 xv[e] = make_float2(Zk.x + Zk.y, Zk.x - Zk.y);

@@ -210,6 +210,21 @@ cudaError_t launch_col_fast_worlds(int H, int M, const FastTables& t, int batch,
 cudaError_t launch_row_fast_worlds(int H, int M, const FastTables& t, const float2* tw_r2c, int batch,
                                    const SpectralWorld* worlds, int n, cudaStream_t s);
 
+// The other lengths with factors 2, 3 and 5 (lenia_fft_wide.cuh: columns 64 to
+// 4096, half rows 32 to 2048), beside the catalogue above: plans of either
+// kind, and launches of one world by shape. Shapes 0 and 1 are a wide length's
+// larger and smaller columns (rows) per CTA; a catalogue length takes its own
+// columns / rows per CTA, as launch_col_fast and launch_row_fast do. Planes of
+// M columns hold padded_spectral_columns(M).
+constexpr int padded_spectral_columns(int M) { return (M + kSpectralBlock - 1) / kSpectralBlock * kSpectralBlock; }
+bool spectral_col_plan(int H, FastPlan& forward_plan);
+bool spectral_row_plan(int M, FastPlan& inverse_plan);
+cudaError_t launch_col_wide(const FftGeometry& g, const FastTables& t, int shape, const float2* S, float2* U,
+                            cudaStream_t s);
+cudaError_t launch_row_wide(const FftGeometry& g, const FastTables& t, int shape, const float2* U, const float* A,
+                            float* A_out, float2* S_next, const StepParams& p, int nk, cudaStream_t s,
+                            void* rgba16f = nullptr, const ColorMapParams* cm = nullptr);
+
 // One persistent launch per substep of a batch (lenia_batch_persistent.cu):
 // CTAs of kPersistThreads claim work items in list order; a row item waits
 // for its world's column items (a counter per world); the last CTA advances

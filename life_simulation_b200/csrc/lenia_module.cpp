@@ -518,7 +518,7 @@ void LeniaModule::release() {
     rel(d_tw_col_);
     rel(d_tw_r2c_);
     for (auto& t : d_fast_tw_) rel(t);
-    fast_col_ = fast_row_ = false;
+    fast_col_ = fast_row_ = wide_ = false;
     fast_ = FastTables();
     d_weights_ = nullptr;
     d_spans_ = nullptr;
@@ -994,7 +994,7 @@ int LeniaModule::buildSpectralTables(const std::vector<KernelDef>& eff) {
         std::copy(spec.begin(), spec.end(), khat.begin() + size_t(k) * (M + 1) * Hh);
     }
     cudaError_t e;
-    const size_t spec = size_t(M) * H;
+    const size_t spec = size_t(padded_spectral_columns(M)) * H;
     if ((e = dev_alloc(&d_S_, spec, device_bytes_)) != cudaSuccess) return cudaFail(e, "cudaMalloc spectrum");
     if ((e = dev_alloc(&d_U_, spec * nk, device_bytes_)) != cudaSuccess) return cudaFail(e, "cudaMalloc potentials");
     if ((e = dev_alloc(&d_khat_, khat.size(), device_bytes_)) != cudaSuccess) return cudaFail(e, "cudaMalloc khat");
@@ -1016,8 +1016,11 @@ int LeniaModule::buildSpectralTables(const std::vector<KernelDef>& eff) {
     // The fast passes share the blocked spectral layout, so they are used
     // together or not at all.
     FastPlan cf, ri;
-    const bool fast = fast_col_plan(H, cf) && fast_row_plan(M, ri) && M % kSpectralBlock == 0;
+    const bool catalogue = fast_col_plan(H, cf) && fast_row_plan(M, ri) && M % kSpectralBlock == 0;
+    const bool fast = catalogue || (spectral_col_plan(H, cf) && spectral_row_plan(M, ri) &&
+                                    std::getenv("LENIA_FFT_RUNTIME_PLAN") == nullptr);
     fast_col_ = fast_row_ = fast;
+    wide_ = fast && !catalogue;
     auto upload_plan = [&](const FastPlan& pl, float2*& dst) -> int {
         std::vector<float2> tw;
         fast_plan_twiddles(pl, tw);
@@ -1054,6 +1057,7 @@ int LeniaModule::buildSpectralTables(const std::vector<KernelDef>& eff) {
 // each candidate on this context's own buffers (contents irrelevant).
 int LeniaModule::autotuneSpectral() {
     if (!fast_col_ && !fast_row_) return LENIA_OK;
+    if (wide_) return autotuneWide();
     cudaEvent_t a = takeEvent(), b = takeEvent();
     StepParams p{};
     p.num_kernels = uint32_t(fgeo_.nk);
@@ -1135,14 +1139,56 @@ int LeniaModule::autotuneSpectral() {
     return LENIA_OK;
 }
 
+// The shapes of the wide lengths' passes: each pass's two timed on this
+// context's own buffers (contents irrelevant), the larger kept unless the
+// smaller is 3 % faster.
+int LeniaModule::autotuneWide() {
+    cudaEvent_t a = takeEvent(), b = takeEvent();
+    StepParams p{};
+    p.num_kernels = uint32_t(fgeo_.nk);
+    p.width = w_;
+    p.height = h_;
+    p.sigma[0] = p.sigma[1] = p.sigma[2] = p.sigma[3] = 1.0f;
+    const auto time_it = [&](auto&& fn) {
+        float best = 1e30f;
+        for (int rep = 0; rep < 5; ++rep) {
+            cudaEventRecord(a, stream_);
+            for (int i = 0; i < 3; ++i)
+                if (fn() != cudaSuccess) return 1e30f;
+            cudaEventRecord(b, stream_);
+            cudaEventSynchronize(b);
+            float ms = 1e30f;
+            cudaEventElapsedTime(&ms, a, b);
+            if (rep > 0) best = std::min(best, ms);
+        }
+        return best;
+    };
+    float col[2], row[2];
+    for (int shape = 0; shape < 2; ++shape)
+        col[shape] = time_it([&] { return launch_col_wide(fgeo_, fast_, shape, d_S_, d_U_, stream_); });
+    col_batch_ = col[1] < 0.97f * col[0] ? 1 : 0;
+    for (int shape = 0; shape < 2; ++shape)
+        row[shape] = time_it([&] {
+            return launch_row_wide(fgeo_, fast_, shape, d_U_, field_[0], field_[1], d_S_, p, fgeo_.nk, stream_);
+        });
+    row_batch_ = row[1] < 0.97f * row[0] ? 1 : 0;
+    cudaGetLastError();
+    if (col[col_batch_] >= 1e29f || row[row_batch_] >= 1e29f) fast_col_ = fast_row_ = wide_ = false;
+    event_pool_.push_back(a);
+    event_pool_.push_back(b);
+    cudaMemsetAsync(field_[0], 0, sizeof(float) * w_ * h_, stream_);
+    cudaMemsetAsync(field_[1], 0, sizeof(float) * w_ * h_, stream_);
+    return LENIA_OK;
+}
+
 void LeniaModule::tuning(int* cols, int* rows) const {
-    const bool on = fast_col_ && fast_row_;
+    const bool on = fast_col_ && fast_row_ && !wide_;
     *cols = on ? col_batch_ : 0;
     *rows = on ? row_batch_ : 0;
 }
 
 int LeniaModule::setTuning(int cols, int rows) {
-    if (!(fast_col_ && fast_row_))
+    if (!(fast_col_ && fast_row_) || wide_)
         return fail(LENIA_ERR_INVALID_ARG, "launch shapes apply to the compile-time-plan spectral passes only");
     if (!fast_shapes_supported(int(h_), int(w_ / 2), cols, rows))
         return fail(LENIA_ERR_INVALID_ARG, "unsupported launch shape: " + std::to_string(cols) + " columns, " +
@@ -1362,22 +1408,26 @@ int LeniaModule::stepImpl(const lenia_frame_params& fp, uint32_t substeps, cudaS
         if (use_fft_) {
             if (!spectrum_valid_) {
                 e = launch(LENIA_PHASE_ROW_FFT, s, [&] {
-                    return fast_row_ ? launch_row_fast(fgeo_, fast_, row_batch_, nullptr, src, nullptr, d_S_, p, 0, s)
-                                     : launch_row_r2c(fgeo_, src, d_S_, s);
+                    return wide_     ? launch_row_wide(fgeo_, fast_, row_batch_, nullptr, src, nullptr, d_S_, p, 0, s)
+                           : fast_row_ ? launch_row_fast(fgeo_, fast_, row_batch_, nullptr, src, nullptr, d_S_, p, 0, s)
+                                       : launch_row_r2c(fgeo_, src, d_S_, s);
                 });
                 if (e != cudaSuccess) return cudaFail(e, "row pass");
             }
             e = launch(LENIA_PHASE_COLUMN, s, [&] {
                 if (tc_precision_ != LENIA_FFT_FP32) return launchColumnTc(tc_batch_, d_S_, d_U_, s);
-                return fast_col_ ? launch_col_fast(fgeo_, fast_, col_batch_, d_S_, d_U_, s)
-                                 : launch_col_conv(fgeo_, d_S_, d_U_, s);
+                return wide_       ? launch_col_wide(fgeo_, fast_, col_batch_, d_S_, d_U_, s)
+                       : fast_col_ ? launch_col_fast(fgeo_, fast_, col_batch_, d_S_, d_U_, s)
+                                   : launch_col_conv(fgeo_, d_S_, d_U_, s);
             });
             if (e != cudaSuccess) return cudaFail(e, "column pass");
             void* out_rgba = i + 1 == n ? rgba16f : nullptr;
             e = launch(LENIA_PHASE_ROW_GROWTH, s, [&] {
-                return fast_row_ ? launch_row_fast(fgeo_, fast_, row_batch_, d_U_, src, dst, d_S_, p, fgeo_.nk, s,
+                return wide_       ? launch_row_wide(fgeo_, fast_, row_batch_, d_U_, src, dst, d_S_, p, fgeo_.nk, s,
                                                    out_rgba, &colormap_)
-                                 : launch_row_c2r_growth(fgeo_, d_U_, src, dst, d_S_, p, s);
+                       : fast_row_ ? launch_row_fast(fgeo_, fast_, row_batch_, d_U_, src, dst, d_S_, p, fgeo_.nk, s,
+                                                     out_rgba, &colormap_)
+                                   : launch_row_c2r_growth(fgeo_, d_U_, src, dst, d_S_, p, s);
             });
             if (e != cudaSuccess) return cudaFail(e, "growth pass");
             spectrum_valid_ = true;

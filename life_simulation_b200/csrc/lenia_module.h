@@ -151,6 +151,7 @@ private:
     int buildDirectTables();
     int buildSpectralTables(const std::vector<KernelDef>& eff);
     int autotuneSpectral();
+    int autotuneWide();
     // The tensor-core column pass: kTcgen05, or mma.sync at `choice` columns per CTA.
     cudaError_t launchColumnTc(int choice, const float2* S, float2* U, cudaStream_t s);
     int stepImpl(const lenia_frame_params& fp, uint32_t substeps, cudaStream_t stream, void* rgba16f);
@@ -216,6 +217,7 @@ private:
     uint32_t direct_taps_ = 0;  // nonzero taps over the direct path's kernels
     FftGeometry fgeo_{};
     bool fast_col_ = false, fast_row_ = false;  // compile-time-plan passes
+    bool wide_ = false;  // the passes of lenia_fft_wide.cuh (col_batch_ / row_batch_ are their shapes)
     int col_batch_ = 2, row_batch_ = 2;         // autotuned per size
     uint32_t tc_precision_ = LENIA_FFT_FP32;    // column DFT stages on the tensor cores
     int tc_batch_ = 2;
