@@ -467,10 +467,10 @@ cudaError_t launch_col_t(const SpectralWorld& w0, const SpectralWorld* worlds, i
     auto fn = col_fast_kernel<PF, B, S>;
     const size_t smem = ColStage<PF, B, S>::smem();
     if (smem > 227 * 1024 || K::T > 1024) return cudaErrorInvalidConfiguration;
-    cudaError_t e = prepare(fn, smem);
-    if (e != cudaSuccess) return e;
+    static KernelState state;
     int per = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, K::T, smem);
+    cudaError_t e = prepare(state, fn, K::T, smem, per);
+    if (e != cudaSuccess) return e;
     return launch_chained(fn, world_grid(per, (M + B - 1) / B, n), K::T, smem, s, w0, worlds, t.col_twf, t.col_twi);
 }
 
@@ -481,10 +481,10 @@ cudaError_t launch_row_t(const SpectralWorld& w0, const SpectralWorld* worlds, i
     auto fn = row_fast_kernel<PI, RB, PIPE, CM, S>;
     const size_t smem = K::smem(PIPE ? 3 : 2);
     if (smem > 227 * 1024) return cudaErrorInvalidConfiguration;
-    cudaError_t e = prepare(fn, smem);
-    if (e != cudaSuccess) return e;
+    static KernelState state;
     int per = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, K::T, smem);
+    cudaError_t e = prepare(state, fn, K::T, smem, per);
+    if (e != cudaSuccess) return e;
     return launch_chained(fn, world_grid(per, (H + RB - 1) / RB, n), K::T, smem, s, w0, worlds, tw_r2c, t.row_twi,
                           t.row_twf);
 }

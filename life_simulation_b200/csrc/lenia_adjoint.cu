@@ -566,10 +566,10 @@ cudaError_t launch_col_adj_t(const AdjColWorld* worlds, int n, const AdjColArgs&
         auto fn = col_adj_kernel<PF, B>;
         const size_t smem = ColAdjK<PF, B>::smem();
         if (smem > 227 * 1024) return cudaErrorInvalidConfiguration;
-        cudaError_t e = prepare(fn, smem);
-        if (e != cudaSuccess) return e;
+        static KernelState state;
         int per = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, K::T, smem);
+        cudaError_t e = prepare(state, fn, K::T, smem, per);
+        if (e != cudaSuccess) return e;
         fn<<<world_grid(per, (args.M + B - 1) / B, n), K::T, smem, s>>>(worlds, args, t.col_twf, t.col_twi);
         return cudaGetLastError();
     }
@@ -585,10 +585,10 @@ cudaError_t launch_row_adj_t(const AdjRowWorld* worlds, int n, const AdjRowArgs&
         auto fn = row_adj_kernel<PI, RB>;
         const size_t smem = K::smem();
         if (smem > 227 * 1024) return cudaErrorInvalidConfiguration;
-        cudaError_t e = prepare(fn, smem);
-        if (e != cudaSuccess) return e;
+        static KernelState state;
         int per = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, K::T, smem);
+        cudaError_t e = prepare(state, fn, K::T, smem, per);
+        if (e != cudaSuccess) return e;
         const int H = int(args.p.height);
         fn<<<world_grid(per, (H + RB - 1) / RB, n), K::T, smem, s>>>(worlds, args, tw_r2c, t.row_twi, t.row_twf);
         return cudaGetLastError();

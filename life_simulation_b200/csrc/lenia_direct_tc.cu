@@ -531,7 +531,9 @@ cudaError_t launch_t(int nk, const float* src, float* dst, const DirectTcPlan& p
                      const uint32_t* spans, const DirectGeometry& g, const StepParams& p, int* err, cudaStream_t s) {
     auto fn = direct_tc_kernel<P>;
     constexpr size_t smem = 6 * size_t(kRows + 2 * P) * (kTX + 2 * P) + size_t(kStages) * kChunk * (1 + P / 16);
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    static fastfft::KernelState state;
+    int per = 0;
+    cudaError_t e = fastfft::prepare(state, fn, kThreads, smem, per);
     if (e != cudaSuccess) return e;
     const int tx = int((p.width + kTX - 1) / kTX), tiles = tx * int((p.height + kRows - 1) / kRows);
     return fastfft::launch_chained(fn, dim3(unsigned(std::min(tiles, fastfft::sms()))), kThreads, smem, s, src, dst,

@@ -154,10 +154,10 @@ cudaError_t launch_t(const SpectralWorld& w0, const SpectralWorld* worlds, int n
     auto fn = col_tc_kernel<PF, B, PREC>;
     const size_t smem = K::smem();
     if (smem > 227 * 1024) return cudaErrorInvalidConfiguration;
-    cudaError_t e = prepare(fn, smem);
-    if (e != cudaSuccess) return e;
+    static KernelState state;
     int per = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, K::T, smem);
+    cudaError_t e = prepare(state, fn, K::T, smem, per);
+    if (e != cudaSuccess) return e;
     fn<<<world_grid(per, (M + B - 1) / B, n), K::T, smem, s>>>(w0, worlds, t.col_twf, t.col_twi);
     return cudaGetLastError();
 }

@@ -502,7 +502,9 @@ template <int PREC, bool PIPE>
 cudaError_t launch_t(const FftGeometry& g, const float2* S, float2* U, int* err, cudaStream_t s) {
     auto fn = col_tc05_kernel<PREC, PIPE>;
     constexpr size_t smem = PIPE ? kSmem + 2 * size_t(kOp) : kSmem;
-    cudaError_t e = prepare(fn, smem);
+    static KernelState state;
+    int per = 0;
+    cudaError_t e = prepare(state, fn, kT, smem, per);
     if (e != cudaSuccess) return e;
     const int groups = g.M / kB;
     const int grid = std::max(1, std::min(groups, sms()));

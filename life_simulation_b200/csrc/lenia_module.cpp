@@ -1259,19 +1259,19 @@ void LeniaModule::reset(uint32_t seed) {
 }
 
 // param(ctx, key, fallback) reads "<instance>.<key>" from the bus
-// (SimulationModule.h:120-123, Lenia.cpp:456-464).
+// (SimulationModule.h:120-123, Lenia.cpp:456-464); the eight keys are spelled
+// out once, in configure.
 lenia_frame_params LeniaModule::resolveFrameParams(const ParameterBus& bus, uint32_t frame_index,
                                                    uint32_t audio_frame) const {
-    const auto param = [&](const char* key, float fallback) { return bus.value(instance_ + "." + key, fallback); };
     lenia_frame_params fp{};
-    fp.dt = param("dt", fallback_dt_);
-    fp.growth_mu = param("growthMu", fallback_mu_);
-    fp.growth_sigma = param("growthSigma", fallback_sigma_);
-    fp.noise_amount = param("noiseAmount", 0.0f);
-    fp.mu_jitter = param("muJitter", 0.0f);
-    fp.inject_amount = param("injectAmount", 0.0f);
-    fp.inject_count = uint32_t(param("injectCount", 3.0f) + 0.5f);
-    fp.growth_mode = uint32_t(param("growthMode", 1.0f) + 0.5f);
+    fp.dt = bus.value(keys_[0], fallback_dt_);
+    fp.growth_mu = bus.value(keys_[1], fallback_mu_);
+    fp.growth_sigma = bus.value(keys_[2], fallback_sigma_);
+    fp.noise_amount = bus.value(keys_[3], 0.0f);
+    fp.mu_jitter = bus.value(keys_[4], 0.0f);
+    fp.inject_amount = bus.value(keys_[5], 0.0f);
+    fp.inject_count = uint32_t(bus.value(keys_[6], 3.0f) + 0.5f);
+    fp.growth_mode = uint32_t(bus.value(keys_[7], 1.0f) + 0.5f);
     fp.frame_index = frame_index;
     fp.audio_frame = audio_frame;
     return fp;

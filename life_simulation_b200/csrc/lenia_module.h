@@ -77,6 +77,9 @@ public:
     // SimulationModule::configure (SimulationModule.h:112-115).
     void configure(std::string instance, ModuleConfig cfg) {
         instance_ = std::move(instance);
+        const char* names[8] = {"dt", "growthMu", "growthSigma", "noiseAmount", "muJitter", "injectAmount",
+                                "injectCount", "growthMode"};
+        for (int i = 0; i < 8; ++i) keys_[i] = instance_ + "." + names[i];
         cfg_ = std::move(cfg);
         colormap_ = cfg_.colormap;
     }
@@ -161,6 +164,7 @@ private:
     void release();
 
     std::string instance_ = "lenia0";
+    std::string keys_[8];  // "<instance>.<key>" of resolveFrameParams' values
     ColorMapParams colormap_ = lenia_default_colormap();
     ModuleConfig cfg_;
     std::string message_;
