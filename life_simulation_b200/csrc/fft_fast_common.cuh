@@ -26,18 +26,60 @@ constexpr int roundup32(int x) { return (x + 31) / 32 * 32; }
 constexpr __host__ __device__ int blocks_of(int M) { return (M + KB - 1) / KB; }
 constexpr __host__ __device__ int padded_columns(int M) { return blocks_of(M) * KB; }
 
-// Smallest pitch >= n with 2*pitch = 8 (mod 32) (in float2): transforms of a
-// batch start 8 banks apart.
-constexpr int row_pitch(int n) {
-    int p = n;
-    while ((2 * p) % 32 != 8) ++p;
+// Row pitch of a batch of B transforms of n elements (float2), even. Shared
+// memory serves an 8-byte access half a warp at a time: 16 / B consecutive
+// elements of each of the B transforms, which cover the 32 banks once when
+// transforms start 32 / B banks apart (an 8-bank start for every B left B = 2
+// with two-way conflicts on every access: 4096 x 4096, three kernels, column
+// pass of two columns 201 -> 184 us, row pass of two rows 194 -> 174 us).
+constexpr int row_pitch(int n, int B = 4) {
+    const int start = B == 2 ? 16 : B == 8 ? 4 : 8;
+    int p = n + (n & 1);
+    if (B == 1) return p;
+    while ((2 * p) % 32 != start) ++p;
     return p;
+}
+
+// Element order of a first pass's output. Its items write R consecutive
+// elements each in 16-byte pairs, eight lanes at a time, and when R is a
+// multiple of 4 those lanes' pairs start on the same few bank quads: two-way
+// conflicts at B = 4, four-way at B = 2, eight-way (R = 16) at one row. So
+// element i goes to i ^ x(i), x a multiple of 2 that differs between the
+// colliding lanes, and the pass that reads it applies the same: x(i) depends
+// on i / R, which the reading items (i = j + t * N / R1, N / R1 a multiple of
+// R) mostly know from j alone. Half-warps of 8-byte reads stay within runs
+// that x permutes, so they are conflict-free as before.
+template <class P, int B>
+struct FirstPassOrder {
+    static constexpr int R = P::radix(0);
+    static constexpr int SHIFT = B == 1 ? 4 : R == 16 ? 4 : R == 8 ? 3 : 2;
+    static constexpr int MASK = B == 1 ? 7 : B == 2 ? 3 : 1;
+    static constexpr int N1 = P::n / P::radix(P::np > 1 ? 1 : 0);  // stride of the reading pass's inputs
+    static constexpr bool on = P::np > 1 && (B == 1 || B == 2 || B == 4) && (R == 4 || R == 8 || R == 16) &&
+                               N1 % (1 << SHIFT) == 0 && P::n % (2 * (MASK + 1)) == 0;  // x stays inside the row
+    // Whether x is the same for all of a reading item's inputs.
+    static constexpr bool fixed = on && (N1 >> SHIFT) % (MASK + 1) == 0;
+    __device__ __forceinline__ static int x(int i) { return on ? ((i >> SHIFT) & MASK) << 1 : 0; }
+};
+// Input t of item j of pass PASS, in the order its buffer holds: pass 1 reads
+// a first pass's output.
+template <class P, int PASS, int B>
+__device__ __forceinline__ int pass_in(int j, int t) {
+    using I = PassIdx<P, PASS>;
+    using O = FirstPassOrder<P, B>;
+    if constexpr (PASS == 1 && O::on) {
+        if constexpr (O::fixed) return (j ^ O::x(j)) + t * I::NR;
+        const int i = j + t * I::NR;
+        return i ^ O::x(i);
+    }
+    return I::in(j, t);
 }
 
 // One Stockham pass over a batch of B transforms: item q -> (b = q % B,
 // j = q / B). All of a thread's items are loaded first, then twiddled,
 // transformed and stored. src(b, i) / dst(b, i, v) address element i of
-// transform b.
+// transform b (of pass 1 in FirstPassOrder, i. e. of a buffer that store_run
+// filled).
 template <class P, int PASS, bool INV, int B, int T, class Src, class Dst>
 __device__ __forceinline__ void pass_gen(Src&& src, Dst&& dst, const float2* __restrict__ tw, int cols) {
     using I = PassIdx<P, PASS>;
@@ -54,7 +96,7 @@ __device__ __forceinline__ void pass_gen(Src&& src, Dst&& dst, const float2* __r
         ok[it] = (TOT % T == 0 || q < TOT) && bi[it] < cols;
         if (ok[it]) {
 #pragma unroll
-            for (int t = 0; t < I::R; ++t) v[it][t] = src(bi[it], I::in(jj[it], t));
+            for (int t = 0; t < I::R; ++t) v[it][t] = src(bi[it], pass_in<P, PASS, B>(jj[it], t));
         }
     }
 #pragma unroll
@@ -69,20 +111,26 @@ __device__ __forceinline__ void pass_gen(Src&& src, Dst&& dst, const float2* __r
     }
 }
 
-// The R outputs of one item of a first pass (span 1) are R consecutive
-// elements of a row: written two at a time (16-byte stores, half the store
-// instructions and shared-memory wavefronts) when R is even.
-// `row + base` must be 16-byte aligned when R is even (shared buffers at
-// even float2 offsets, even pitches, base a multiple of R).
-template <int R>
-__device__ __forceinline__ void store_run(float2* row, int base, const float2* v) {
+// The R outputs of item j of plan P's first pass (span 1) are the R
+// consecutive elements from j * R on: written two at a time (16-byte stores,
+// half the store instructions and shared-memory wavefronts) when R is even, in
+// FirstPassOrder. `row` must be 16-byte aligned when R is even (shared buffers
+// at even float2 offsets, even pitches).
+template <class P, int B>
+__device__ __forceinline__ void store_run(float2* row, int j, const float2* v) {
+    using O = FirstPassOrder<P, B>;
+    constexpr int R = P::radix(0);
     if constexpr (R % 2 == 0) {
-        float4* d = reinterpret_cast<float4*>(row + base);
+        // An item's R elements share x: 2t ^ x within its (aligned) run, or
+        // the whole run moved when x reaches past it (R = 4 or 8 at one row).
+        const int base = j * R, x = O::x(base);
 #pragma unroll
-        for (int t = 0; t < R / 2; ++t) d[t] = make_float4(v[2 * t].x, v[2 * t].y, v[2 * t + 1].x, v[2 * t + 1].y);
+        for (int t = 0; t < R / 2; ++t)
+            *reinterpret_cast<float4*>(row + ((base + 2 * t) ^ x)) =
+                make_float4(v[2 * t].x, v[2 * t].y, v[2 * t + 1].x, v[2 * t + 1].y);
     } else {
 #pragma unroll
-        for (int t = 0; t < R; ++t) row[base + t] = v[t];
+        for (int t = 0; t < R; ++t) row[j * R + t] = v[t];
     }
 }
 
@@ -112,7 +160,7 @@ __device__ __forceinline__ void pass0_buf(Src&& src, float2* buf, int cols) {
     for (int it = 0; it < ITEMS; ++it) {
         if (ok[it]) {
             Dft<I::R, INV>::run(v[it]);
-            store_run<I::R>(buf + bi[it] * PITCH, jj[it] * I::R, v[it]);
+            store_run<P, B>(buf + bi[it] * PITCH, jj[it], v[it]);
         }
     }
 }
@@ -162,7 +210,7 @@ struct ColK {
     static constexpr int NRL = H / RL;
     static constexpr int T = roundup32((B * NRL + S - 1) / S);
     static constexpr int ITL = (B * NRL + T - 1) / T;
-    static constexpr int PITCH = row_pitch(H);
+    static constexpr int PITCH = row_pitch(H, B);
     // The work buffers start after the twiddle tables at an even float2
     // offset (16-byte aligned, for store_run's paired stores).
     static constexpr int BUF0 = (PF::tw_size() + PI::tw_size() + 1) / 2 * 2;
@@ -180,7 +228,7 @@ struct RowK {
     static constexpr int NRC = M / RC;
     static constexpr int T = roundup32((RB * NRC + S - 1) / S);
     static constexpr int ITL = (RB * NRC + T - 1) / T;
-    static constexpr int PITCH = row_pitch(padded_columns(M));  // even: rows start 16-byte aligned
+    static constexpr int PITCH = row_pitch(padded_columns(M), RB);  // even: rows start 16-byte aligned
     // Twiddle tables, then the buffers from an even float2 offset so the
     // 16-byte cp.async destinations are 16-byte aligned.
     static constexpr int TABLES = (M + 1) + PI::tw_size() + PF::tw_size();

@@ -167,7 +167,8 @@ __global__ void __launch_bounds__(ColK<PF, B, SPLIT>::T)
         for (int it = 0; it < K::ITL; ++it) {
             if (ok[it]) {
 #pragma unroll
-                for (int t = 0; t < RL; ++t) C[it][t] = X[bi[it] * PITCH + IL::in(jj[it], t)];
+                for (int t = 0; t < RL; ++t)
+                    C[it][t] = X[bi[it] * PITCH + pass_in<PF, PF::np - 1, B>(jj[it], t)];
                 IL::template twiddle<false>(C[it], jj[it], twf);
                 Dft<RL, false>::run(C[it]);
                 if (k0 == 0 && bi[it] == 0) {
@@ -208,7 +209,7 @@ __global__ void __launch_bounds__(ColK<PF, B, SPLIT>::T)
                     }
                 }
                 Dft<RL, true>::run(D);
-                store_run<RL>(Y + bi[it] * PITCH, jj[it] * RL, D);
+                store_run<PI, B>(Y + bi[it] * PITCH, jj[it], D);
             }
             if (kk + 1 < nk) fetch_k(kk + 1);
         };
@@ -371,7 +372,7 @@ __global__ void __launch_bounds__(RowK<PI, RB, SPLIT>::T,
                 if (!ok[it]) continue;
                 float2 z[RC];
 #pragma unroll
-                for (int t = 0; t < RC; ++t) z[t] = X[bi[it] * PITCH + IL::in(jj[it], t)];
+                for (int t = 0; t < RC; ++t) z[t] = X[bi[it] * PITCH + pass_in<PI, PI::np - 1, RB>(jj[it], t)];
                 IL::template twiddle<true>(z, jj[it], twi);
                 Dft<RC, true>::run(z);
                 const uint32_t gy = uint32_t(y0 + bi[it]);
@@ -437,7 +438,7 @@ __global__ void __launch_bounds__(RowK<PI, RB, SPLIT>::T,
         for (int it = 0; it < K::ITL; ++it) {
             if (!ok[it]) continue;
             Dft<RC, false>::run(za[it]);
-            store_run<RC>(bw + bi[it] * PITCH, jj[it] * RC, za[it]);
+            store_run<PF, RB>(bw + bi[it] * PITCH, jj[it], za[it]);
         }
         __syncthreads();
         float2* Y = mid_passes<PF, 1, PF::np - 1, false, RB, T, PITCH>(bw, sA, twf, rows);

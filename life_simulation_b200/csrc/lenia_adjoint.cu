@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(RowK<PI, RB>::T, (512 / RowK<PI, RB>::T > 1 ? 
                 if (!ok[it]) continue;
                 float2 z[RC];
 #pragma unroll
-                for (int t = 0; t < RC; ++t) z[t] = X[bi[it] * PITCH + IL::in(jj[it], t)];
+                for (int t = 0; t < RC; ++t) z[t] = X[bi[it] * PITCH + pass_in<PI, PI::np - 1, RB>(jj[it], t)];
                 IL::template twiddle<true>(z, jj[it], twi);
                 Dft<RC, true>::run(z);
 #pragma unroll
@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(RowK<PI, RB>::T, (512 / RowK<PI, RB>::T > 1 ? 
             for (int it = 0; it < ITL; ++it) {
                 if (!ok[it]) continue;
                 Dft<RC, false>::run(zq[it]);
-                store_run<RC>(ba + bi[it] * PITCH, jj[it] * RC, zq[it]);
+                store_run<PF, RB>(ba + bi[it] * PITCH, jj[it], zq[it]);
             }
             __syncthreads();
             float2* Y = mid_passes<PF, 1, PF::np - 1, false, RB, T, PITCH>(ba, bb, twf, rows);
@@ -456,7 +456,8 @@ __global__ void __launch_bounds__(ColK<PF, B>::T)
             for (int it = 0; it < ITL; ++it) {
                 if (!ok[it]) continue;
 #pragma unroll
-                for (int t = 0; t < RL; ++t) C[it][t] = X[bi[it] * PITCH + IL::in(jj[it], t)];
+                for (int t = 0; t < RL; ++t)
+                    C[it][t] = X[bi[it] * PITCH + pass_in<PF, PF::np - 1, B>(jj[it], t)];
                 IL::template twiddle<false>(C[it], jj[it], twf);
                 Dft<RL, false>::run(C[it]);
                 if (k0 == 0 && bi[it] == 0) {
@@ -544,7 +545,7 @@ __global__ void __launch_bounds__(ColK<PF, B>::T)
         for (int it = 0; it < ITL; ++it) {
             if (!ok[it]) continue;
             Dft<RL, true>::run(G[it]);
-            store_run<RL>(ba + bi[it] * PITCH, jj[it] * RL, G[it]);
+            store_run<PI, B>(ba + bi[it] * PITCH, jj[it], G[it]);
         }
         __syncthreads();
         float2* Z = mid_passes<PI, 1, PI::np - 1, true, B, T, PITCH>(ba, bb, twi, cols);
@@ -933,8 +934,9 @@ cudaError_t row_spectrum(lenia_adjoint* a, int j, cudaStream_t s) {
 }
 
 // Columns per CTA iteration of the forward column pass and rows of the row
-// pass: each candidate timed (CUDA events, after one warm-up launch) on step
-// 0's tables over zeroed buffers; the fastest is kept.
+// pass: each candidate timed (CUDA events, the least of three pairs of launches
+// after one warm-up launch; a single pair's spread is wider than the shapes'
+// differences) on step 0's tables over zeroed buffers; the fastest is kept.
 cudaError_t autotune(lenia_adjoint* a) {
     const cudaStream_t s = a->stream;
     cudaError_t e = cudaMemsetAsync(a->ckpt, 0, sizeof(float) * a->nb * a->P, s);
@@ -948,11 +950,16 @@ cudaError_t autotune(lenia_adjoint* a) {
     const auto timed = [&](auto launch, float* ms) -> cudaError_t {
         cudaError_t r = launch();
         if (r != cudaSuccess) return r;
-        cudaEventRecord(t0, s);
-        for (int i = 0; i < 3 && r == cudaSuccess; ++i) r = launch();
-        cudaEventRecord(t1, s);
-        if (r == cudaSuccess) r = cudaEventSynchronize(t1);
-        if (r == cudaSuccess) r = cudaEventElapsedTime(ms, t0, t1);
+        *ms = 1e30f;
+        for (int rep = 0; rep < 3 && r == cudaSuccess; ++rep) {
+            cudaEventRecord(t0, s);
+            for (int i = 0; i < 2 && r == cudaSuccess; ++i) r = launch();
+            cudaEventRecord(t1, s);
+            if (r == cudaSuccess) r = cudaEventSynchronize(t1);
+            float t = 0.0f;
+            if (r == cudaSuccess) r = cudaEventElapsedTime(&t, t0, t1);
+            if (r == cudaSuccess) *ms = std::min(*ms, t);
+        }
         return r;
     };
     float best = 1e30f;

@@ -103,7 +103,7 @@ template <class PF, int B>
 struct PCol {
     using PI = typename Reverse<PF>::type;
     static constexpr int H = PF::n, RL = PF::last(), NRL = H / RL, Hh = H / 2 + 1;
-    static constexpr int PITCH = row_pitch(H);
+    static constexpr int PITCH = row_pitch(H, B);
     static constexpr int ITL = (B * NRL + kPT - 1) / kPT;
     static constexpr size_t smem = sizeof(float2) * (2 * size_t(B) * PITCH + H);
 };
@@ -111,7 +111,7 @@ template <class PI, int RB>
 struct PRow {
     using PF = typename Reverse<PI>::type;
     static constexpr int M = PI::n, RC = PI::last(), NRC = M / RC;
-    static constexpr int PITCH = row_pitch(M);
+    static constexpr int PITCH = row_pitch(M, RB);
     static constexpr int ITL = (RB * NRC + kPT - 1) / kPT;
     static constexpr size_t smem = sizeof(float2) * 3 * size_t(RB) * PITCH;
 };
@@ -150,8 +150,7 @@ __device__ __noinline__ void col_item(const SpectralWorld& sw, int k0, const flo
         ok[it] = q < B * NRL && bi[it] < cols;
     }
     // S was written by the previous launch's row items; loads at L2.
-    pass_gen<PF, 0, false, B, kPT>([&](int b, int i) { return __ldcg(S + at(b, i)); },
-                                   [&](int b, int i, float2 v) { ba[b * PITCH + i] = v; }, twf, cols);
+    pass0_buf<PF, false, B, kPT, PITCH>([&](int b, int i) { return __ldcg(S + at(b, i)); }, ba, cols);
     __syncthreads();
     float2* X = mid_passes<PF, 1, PF::np - 1, false, B, kPT, PITCH>(ba, bb, twf, cols);
     float2* Y = (PF::np - 2) % 2 ? ba : bb;
@@ -160,7 +159,7 @@ __device__ __noinline__ void col_item(const SpectralWorld& sw, int k0, const flo
     for (int it = 0; it < ITL; ++it) {
         if (ok[it]) {
 #pragma unroll
-            for (int t = 0; t < RL; ++t) C[it][t] = X[bi[it] * PITCH + IL::in(jj[it], t)];
+            for (int t = 0; t < RL; ++t) C[it][t] = X[bi[it] * PITCH + pass_in<PF, PF::np - 1, B>(jj[it], t)];
             IL::template twiddle<false>(C[it], jj[it], twf);
             Dft<RL, false>::run(C[it]);
             if (k0 == 0 && bi[it] == 0) {
@@ -191,8 +190,7 @@ __device__ __noinline__ void col_item(const SpectralWorld& sw, int k0, const flo
                 }
             }
             Dft<RL, true>::run(D);
-#pragma unroll
-            for (int t = 0; t < RL; ++t) Y[bi[it] * PITCH + jj[it] * RL + t] = D[t];
+            store_run<PI, B>(Y + bi[it] * PITCH, jj[it], D);
         }
     };
     const auto last_inverse = [&](int kk, const float2* Z) {
@@ -260,8 +258,7 @@ __device__ __noinline__ void row_item(const SpectralWorld& sw, int y0, const flo
             cp_async_wait_all();
         }
         __syncthreads();
-        pass_gen<PI, 0, true, RB, kPT>([&](int b, int i) { return c2r_split<M>(sU + b * PITCH, twr, i); },
-                                       [&](int b, int i, float2 v) { bw[b * PITCH + i] = v; }, twi, rows);
+        pass0_buf<PI, true, RB, kPT, PITCH>([&](int b, int i) { return c2r_split<M>(sU + b * PITCH, twr, i); }, bw, rows);
         __syncthreads();
         float2* X = mid_passes<PI, 1, PI::np - 1, true, RB, kPT, PITCH>(bw, sU, twi, rows);
         const auto pick = [&](const float(&a)[kMaxKernels]) {
@@ -273,7 +270,7 @@ __device__ __noinline__ void row_item(const SpectralWorld& sw, int y0, const flo
             if (!ok[it]) continue;
             float2 z[RC];
 #pragma unroll
-            for (int t = 0; t < RC; ++t) z[t] = X[bi[it] * PITCH + IL::in(jj[it], t)];
+            for (int t = 0; t < RC; ++t) z[t] = X[bi[it] * PITCH + pass_in<PI, PI::np - 1, RB>(jj[it], t)];
             IL::template twiddle<true>(z, jj[it], twi);
             Dft<RC, true>::run(z);
 #pragma unroll
@@ -314,8 +311,7 @@ __device__ __noinline__ void row_item(const SpectralWorld& sw, int y0, const flo
     for (int it = 0; it < ITL; ++it) {
         if (!ok[it]) continue;
         Dft<RC, false>::run(za[it]);
-#pragma unroll
-        for (int t = 0; t < RC; ++t) bw[bi[it] * PITCH + jj[it] * RC + t] = za[it][t];
+        store_run<PF, RB>(bw + bi[it] * PITCH, jj[it], za[it]);
     }
     __syncthreads();
     float2* Y = mid_passes<PF, 1, PF::np - 1, false, RB, kPT, PITCH>(bw, sA, twf, rows);
