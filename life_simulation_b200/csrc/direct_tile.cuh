@@ -98,13 +98,53 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
 // device stops delivering it).
 constexpr uint32_t kTmaPolls = 1u << 22;
 
+// Rows by .. by + TR - 1, columns bx .. bx + TP - 1 of the torus into tile
+// [TR][TP]. A warp takes eight rows at a time and its lanes walk the columns:
+// the wrapped row starts are found once for the eight rows, a column is
+// wrapped by a subtraction, and eight loads are in flight. (An element at a
+// time -- a division by the pitch and two remainders each -- was most of a
+// small tile's life: see launch_direct_worlds.)
+template <int NT>
+__device__ __forceinline__ void stage_wrapped(float* tile, int TR, int TP, const float* __restrict__ src, int bx, int by,
+                                              int W, int H) {
+    constexpr int ROWS = 8;
+    const int lane = int(threadIdx.x) & 31, warp = int(threadIdx.x) >> 5;
+    int gx0 = (bx + lane) % W;
+    if (gx0 < 0) gx0 += W;
+    const int hop = W > 32 ? 32 : 32 % W;  // 32 columns on, modulo W
+    for (int r0 = warp * ROWS; r0 < TR; r0 += (NT / 32) * ROWS) {
+        const float* row[ROWS];
+        int gy = (by + r0) % H;
+        if (gy < 0) gy += H;
+#pragma unroll
+        for (int q = 0; q < ROWS; ++q) {
+            row[q] = src + size_t(gy) * W;
+            gy = gy + 1 == H ? 0 : gy + 1;
+        }
+        int gx = gx0;
+        for (int c = lane; c < TP; c += 32) {
+            float v[ROWS];
+#pragma unroll
+            for (int q = 0; q < ROWS; ++q) v[q] = __ldg(row[q] + gx);
+#pragma unroll
+            for (int q = 0; q < ROWS; ++q)
+                if (r0 + q < TR) tile[(r0 + q) * TP + c] = v[q];
+            gx += hop;
+            if (gx >= W) gx -= W;
+        }
+    }
+}
+
 // One output tile at (x0, y0) of one world. `tmap` (or null): the state's
 // halo-tile tensor map; `err` counts halo loads whose wait ran out. S > 1
 // splits the kernel rows over S thread groups (group s takes rows dy = s,
 // s + S, ...) for fields too small to fill the GPU one thread per 8 outputs:
 // the groups' partial sums meet in shared memory and are added in group
-// order before the epilogue.
-template <int TW, int TH, int NK, int S = 1, int OX = PX, int OY = 1>
+// order before the epilogue. IEEE (one kernel): the growth map with a division
+// by sigma and the full-range exponential, as a batch's worlds take it: a sweep
+// runs thousands of substeps, over which its fields amplify a last-place
+// difference, and the map is a small part of a batch tile.
+template <int TW, int TH, int NK, int S = 1, int OX = PX, int OY = 1, bool IEEE = false>
 __device__ __forceinline__ void direct_tile(const float* __restrict__ src, float* __restrict__ dst,
                                             const float* __restrict__ weights,  // [NK][2R+1][WP], zero padded
                                             const uint32_t* __restrict__ spans, // [NK][2R+1]
@@ -145,16 +185,7 @@ __device__ __forceinline__ void direct_tile(const float* __restrict__ src, float
             tma_load_2d(tile, tmap, bx, by, &tma_bar);
         }
     } else {
-        for (int i = tid; i < TR * TP; i += NT) {
-            int r = i / TP, c = i - r * TP;
-            int gy = y0 - g.r + r;
-            int gx = x0 - g.xp + c;
-            gy %= H;
-            if (gy < 0) gy += H;
-            gx %= W;
-            if (gx < 0) gx += W;
-            tile[i] = __ldg(src + size_t(gy) * W + gx);
-        }
+        stage_wrapped<NT>(tile, TR, TP, src, bx, by, W, H);
     }
     const int nw = NK * g.ksize * g.wp;
     for (int i = tid; i < nw; i += NT) wts[i] = __ldg(weights + i);
@@ -290,6 +321,22 @@ __device__ __forceinline__ void direct_tile(const float* __restrict__ src, float
         const int gy = y0 + ty + o;
         if (gy >= H) return;
         const float* arow = tile + (ty + o + g.r) * TP + ox + g.xp;
+        float v[OX];
+        if constexpr (IEEE) {
+            static_assert(NK == 1, "one kernel per world");
+#pragma unroll
+            for (int j = 0; j < OX; ++j) {
+                const float mu = p.mu_jitter > 0.0f
+                                     ? p.mu[0] + mu_jitter_shift(p, uint32_t(x0 + ox + j), rand_row(uint32_t(gy), ex.jitter_base))
+                                     : p.mu[0];
+                const float t = (acc[o][0][j] - mu) / p.sigma[0];
+                const float b = expf(-0.5f * t * t), h = p.weight[0], A = arow[j];
+                if (euler.asym)
+                    v[j] = A + p.dt * ((euler.weighted ? h * b / p.sum_weights : A) - A);
+                else
+                    v[j] = A + p.dt * (h * (2.0f * b - 1.0f));
+            }
+        } else {
         float2 sum[OX / 2];  // growth sums of pixel pairs
 #pragma unroll
         for (int k = 0; k < NK; ++k) {
@@ -303,11 +350,11 @@ __device__ __forceinline__ void direct_tile(const float* __restrict__ src, float
                 sum[j] = k == 0 ? c : __fadd2_rn(sum[j], c);
             }
         }
-        float v[OX];
 #pragma unroll
         for (int j = 0; j < OX / 2; ++j) {
             v[2 * j] = euler(arow[2 * j], sum[j].x);
             v[2 * j + 1] = euler(arow[2 * j + 1], sum[j].y);
+        }
         }
         noise_inject_clip(p, ex, v, uint32_t(x0 + ox), uint32_t(gy));
 #pragma unroll

@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(DirectTile<TW, TH>::kThreads)
     const int3 t = tiles[blockIdx.x];
     if (threadIdx.x == 0) w = worlds[t.x];
     __syncthreads();
-    direct_tile<TW, TH, 1>(w.src, w.dst, w.weights, w.spans, w.g, w.p, t.y * TW, t.z * TH, nullptr, nullptr);
+    direct_tile<TW, TH, 1, 1, PX, 1, true>(w.src, w.dst, w.weights, w.spans, w.g, w.p, t.y * TW, t.z * TH, nullptr, nullptr);
 }
 
 template <int TW, int TH, int NK, int S, int OX, int OY>
@@ -206,6 +206,11 @@ bool direct_tma_encode(int tile_cfg, const DirectGeometry& g, float* const field
 cudaError_t launch_direct_worlds(const DirectWorld* worlds, const int3* tiles, int ntiles, int max_r,
                                  cudaStream_t stream) {
     // 32x16 tiles (small worlds); shared memory sized for the largest radius.
+    // A tile's 64 threads stage a halo of up to 80 x 108 values: with a
+    // division and two remainders per value that was as long as the taps. 60
+    // substeps before / with whole rows per warp (stage_wrapped): one world
+    // 128 x 128 R = 8 1022 / 600 us, 512 x 512 R = 12 1594 / 1116 us; 48 worlds
+    // 512 x 512 R = 12 29965 / 23156 us.
     constexpr int TW = 32, TH = 16;
     DirectGeometry g;
     g.r = max_r;
