@@ -299,9 +299,10 @@ int lenia_step_render(lenia_ctx* ctx, const lenia_frame_params* fp, uint32_t sub
  * with spectral worlds; creation times both and keeps the faster
  * (lenia_batch_launch_form). lenia_batch_step replays k substeps as one
  * captured CUDA graph. The path of
- * each world is chosen at creation: LENIA_BATCH_AUTO times the direct and
- * spectral passes on the batch's own buffers and gives each world the
- * cheaper one. Each world evolves exactly as it would alone. */
+ * each world is chosen at creation: LENIA_BATCH_AUTO gives each world the
+ * path whose launches cost it less, by a rule on the batch's sizes and taps
+ * (the same for every batch of the same worlds). Each world evolves exactly
+ * as it would alone. */
 typedef struct lenia_world {
     uint32_t width, height;
     uint32_t radius;          /* kernel radius (px) */

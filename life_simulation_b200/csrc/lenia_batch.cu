@@ -3,7 +3,7 @@
 // the reference sweeps variants one SceneRunner at a time,
 // Apps/LifePresetLab/main.cpp:718-795).
 //
-// Two launch forms of a substep, whichever the autotuner measures faster:
+// Two launch forms of a substep, whichever is measured faster at creation:
 //   * persistent (lenia_batch_persistent.cu): ONE launch over a device work
 //     list of every world's column groups, direct tiles and row groups; row
 //     groups wait on per-world counters for their world's column groups, and
@@ -21,9 +21,8 @@
 // Worlds never interact; a world's result is the same as stepping it alone
 // through a single-world context.
 //
-// Path choice (the autotuner): at creation the direct kernel's cost per
-// pixel-tap and each size's spectral-step cost per pixel are measured on the
-// batch's own buffers; each world takes the cheaper path for its radius.
+// Path choice (policy AUTO): a world takes the path whose launches cost it
+// less, by a rule on sizes and taps (lenia_batch_create).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -654,79 +653,37 @@ int lenia_batch_create(const lenia_world* worlds, uint32_t n, uint32_t policy, l
             return LENIA_OK;
         };
 
-        // Autotuner (policy AUTO): time the batched direct launch over every
-        // direct candidate (cost per pixel-tap) and each class's spectral step
-        // over all its candidates (cost per pixel) -- the batch's own launch
-        // shapes, on its own buffers -- and give each world the cheaper path.
+        // Policy AUTO: the path whose launches, each on its own, cost a world
+        // less -- the spectral step of its size class, shared by the class's
+        // worlds, against its share by pixel-taps of the direct launch over
+        // every world that has both paths. The three constants are fitted to
+        // what timing those launches at creation picked (3456 worlds in
+        // batches of 1 to 60: 97 % the same; timing disagreed with itself on
+        // 1 % between two processes): 6 us a class's two spectral launches,
+        // 40 fs a pixel-tap of a full direct launch, and a direct launch no
+        // shorter than 19 us and 6.3 ns per tap of its largest kernel.
+        // A rule instead of the timing gives a batch the same paths, and so the
+        // same bits, every time. It deliberately keeps the line where the timing
+        // had it, since such fields amplify the two paths' rounding (2e-4 after
+        // 60 substeps on 1 world in 500); for small batches of mixed sizes the
+        // chains run side by side and LENIA_BATCH_FFT is the faster policy
+        // (4 worlds x 60 substeps 1.1 against 1.8 to 2.4 ms, 8 worlds 1.2 against
+        // 1.9 to 4.2; from 48 worlds on they are level).
         if (policy == LENIA_BATCH_AUTO) {
-            cudaEvent_t ea, eb;
-            cudaEventCreate(&ea);
-            cudaEventCreate(&eb);
-            auto time_ms = [&](auto&& fn) {
-                float best = 1e30f;
-                for (int rep = 0; rep < 3; ++rep) {
-                    cudaEventRecord(ea, b.stream);
-                    if (fn() != cudaSuccess) return 1e30f;
-                    cudaEventRecord(eb, b.stream);
-                    cudaEventSynchronize(eb);
-                    float ms = 0.0f;
-                    cudaEventElapsedTime(&ms, ea, eb);
-                    if (rep > 0) best = std::min(best, ms);
-                }
-                return best;
-            };
-            // Cost per tap of the batched direct launch over every candidate.
-            // That launch sizes its halo tile for the largest radius it holds,
-            // which overstates the cost for small radii; so candidates are also
-            // timed in radius bands, each with its own halo, and a band with
-            // enough work (>= 1e8 pixel-taps, so the launch itself is amortised)
-            // uses its own figure.
-            const auto band = [&](uint32_t i) { return worlds[i].radius <= 12u ? 0 : worlds[i].radius <= 20u ? 1 : 2; };
-            std::vector<int> dall, dcand[3];
-            double taps_all = 0.0, taps[3] = {0.0, 0.0, 0.0};
+            constexpr double kClass = 6e-6, kTap = 40e-15, kDirect = 19e-6, kLargest = 6.3e-9;
+            const auto taps = [&](uint32_t i) { return double(worlds[i].width) * worlds[i].height * nnz[i]; };
+            double total = 0.0;
+            uint32_t largest = 0;
             for (uint32_t i = 0; i < n; ++i)
                 if (can_direct[i] && can_fft[i]) {
-                    const double t = double(worlds[i].width) * worlds[i].height * nnz[i];
-                    dall.push_back(int(i));
-                    dcand[band(i)].push_back(int(i));
-                    taps_all += t;
-                    taps[band(i)] += t;
+                    total += taps(i);
+                    largest = std::max(largest, nnz[i]);
                 }
-            const auto time_direct = [&](const std::vector<int>& ids, double t, double& out) {
-                DirectWorld* dt[2] = {nullptr, nullptr};
-                int3* tl = nullptr;
-                int nt = 0, mr = 0;
-                if (build_direct(ids, dt, &tl, &nt, &mr) < 0) return false;
-                const float ms = time_ms([&] { return launch_direct_worlds(dt[0], tl, nt, mr, b.stream); });
-                out = double(ms) / t;
-                return true;
-            };
-            double cost_all = 0.0, cost_tap[3] = {0.0, 0.0, 0.0};
-            if (!dall.empty() && !time_direct(dall, taps_all, cost_all)) return LENIA_ERR_CUDA;
-            for (int bd = 0; bd < 3; ++bd) {
-                cost_tap[bd] = cost_all;
-                if (taps[bd] >= 1e8 && !time_direct(dcand[bd], taps[bd], cost_tap[bd])) return LENIA_ERR_CUDA;
-            }
-            std::vector<double> cost_px(b.classes.size(), 0.0);
-            for (size_t ci = 0; ci < b.classes.size(); ++ci) {
-                auto& c = b.classes[ci];
-                SpectralWorld* st[2] = {nullptr, nullptr};
-                SpectralWorld* rt[2] = {nullptr, nullptr};
-                if (build_spectral(ci, class_members[ci], st, rt) < 0) return LENIA_ERR_CUDA;
-                const int cnt = int(class_members[ci].size());
-                const float ms = time_ms([&] {
-                    cudaError_t r = launch_col_fast_worlds(c.H, c.M, c.t, c.col_batch, st[0], cnt, b.stream);
-                    if (r == cudaSuccess) r = launch_row_fast_worlds(c.H, c.M, c.t, c.tw_r2c, c.row_batch, st[0], cnt, b.stream);
-                    return r;
-                });
-                cost_px[ci] = double(ms) / (double(c.W) * c.H * cnt);
-            }
-            cudaEventDestroy(ea);
-            cudaEventDestroy(eb);
+            const double per_tap = total > 0.0 ? std::max(kTap, (kDirect + kLargest * largest) / total) : kTap;
             for (uint32_t i = 0; i < n; ++i)
                 if (can_direct[i] && can_fft[i])
-                    b.path[i] = (cost_tap[band(i)] * nnz[i] <= cost_px[size_t(cls[i])]) ? LENIA_CONV_DIRECT : LENIA_CONV_FFT;
-            cudaMemsetAsync(b.fields, 0, total * sizeof(float), b.stream);
+                    b.path[i] = taps(i) * per_tap <= kClass / double(class_members[size_t(cls[i])].size()) ? LENIA_CONV_DIRECT
+                                                                                                      : LENIA_CONV_FFT;
         }
 
         // Final tables.
@@ -844,20 +801,29 @@ int lenia_batch_create(const lenia_world* worlds, uint32_t n, uint32_t policy, l
                 cudaEventCreate(&ea);
                 cudaEventCreate(&eb);
                 float ms[2] = {0.0f, 0.0f};
+                // Four substeps of each as they run, in a captured graph (in
+                // plain streams the per-size form's launches wait for the host).
                 for (int form = 0; form < 2; ++form) {
                     b.persistent = form == 1;
-                    float best = 1e30f;
-                    for (int rep = 0; rep < 4; ++rep) {
-                        cudaEventRecord(ea, b.stream);
-                        const cudaError_t r = b.launch_steps(0, 4, b.stream, false);
-                        cudaEventRecord(eb, b.stream);
-                        cudaEventSynchronize(eb);
-                        float t = 0.0f;
-                        cudaEventElapsedTime(&t, ea, eb);
-                        if (r != cudaSuccess) t = 1e30f;
-                        if (rep > 0) best = std::min(best, t);
+                    ms[form] = 1e30f;
+                    cudaGraph_t graph = nullptr;
+                    cudaGraphExec_t exec = nullptr;
+                    if (cudaStreamBeginCapture(b.stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) continue;
+                    const cudaError_t r = b.launch_steps(0, 4, b.stream, false);
+                    const cudaError_t r2 = cudaStreamEndCapture(b.stream, &graph);
+                    if (r == cudaSuccess && r2 == cudaSuccess && cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess) {
+                        for (int rep = 0; rep < 4; ++rep) {
+                            cudaEventRecord(ea, b.stream);
+                            const cudaError_t l = cudaGraphLaunch(exec, b.stream);
+                            cudaEventRecord(eb, b.stream);
+                            cudaEventSynchronize(eb);
+                            float t = 1e30f;
+                            if (l == cudaSuccess && cudaEventElapsedTime(&t, ea, eb) == cudaSuccess && rep > 0)
+                                ms[form] = std::min(ms[form], t);
+                        }
+                        cudaGraphExecDestroy(exec);
                     }
-                    ms[form] = best;
+                    if (graph) cudaGraphDestroy(graph);
                 }
                 cudaEventDestroy(ea);
                 cudaEventDestroy(eb);
