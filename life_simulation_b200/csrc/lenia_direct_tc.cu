@@ -67,6 +67,7 @@ constexpr int kThreads = 32 * 19;
 constexpr int kStages = 6;             // T blocks in flight
 constexpr uint32_t kCols = 512;        // tensor-memory columns: per buffer and issuing warp 128 (four levels)
 constexpr uint32_t kChunk = 96u * 32u; // bytes of one chunk's T: 96 rows of 32 k
+constexpr int kTurn = kPart + 4;       // pitch (floats) of the rows an epilogue warp turns A and A' in
 constexpr uint32_t kPolls = 1u << 20;  // polls of a barrier before a CTA gives up (about a second)
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -175,6 +176,23 @@ __device__ __forceinline__ int wrap(int v, int n) {
     return v < 0 ? v + n : v;
 }
 
+// 0 <= a < 2 exactly when the sign and the top exponent bit are clear (-0
+// takes the FP32 form as well).
+__device__ __forceinline__ bool out_of_range(const float4& a) {
+    return (((__float_as_uint(a.x) | __float_as_uint(a.y)) | (__float_as_uint(a.z) | __float_as_uint(a.w))) &
+            0xC0000000u) != 0u;
+}
+// Four values as the bytes of levels 0, 1 and 2, value i in byte i.
+__device__ __forceinline__ void pack_bytes(const float4& a, uint32_t (&w)[3]) {
+    const uint32_t v0 = __float2uint_rn(a.x * 8388608.0f), v1 = __float2uint_rn(a.y * 8388608.0f);
+    const uint32_t v2 = __float2uint_rn(a.z * 8388608.0f), v3 = __float2uint_rn(a.w * 8388608.0f);
+    const uint32_t l01 = __byte_perm(v0, v1, 0x5140), l23 = __byte_perm(v2, v3, 0x5140);
+    const uint32_t h01 = __byte_perm(v0, v1, 0x7362), h23 = __byte_perm(v2, v3, 0x7362);
+    w[0] = __byte_perm(h01, h23, 0x5410);
+    w[1] = __byte_perm(l01, l23, 0x7632);
+    w[2] = __byte_perm(l01, l23, 0x5410);
+}
+
 // One output of the FP32 form (values the byte form cannot hold): taps in
 // the order of direct_tile.
 __device__ __noinline__ float direct_point(const float* __restrict__ src, const float* __restrict__ weights,
@@ -279,6 +297,42 @@ __global__ void __launch_bounds__(kThreads, 1)
             const bool inside = W % 4 == 0 && x0 >= P && x0 + kTX + P <= W;
             unsigned char* planes = sm + buf * 3u * kPlane;
             bool bad = false;
+            if (W % 4 != 0 && x0 >= P && x0 + kTX + P + 3 <= W) {
+                // Rows start anywhere in a 16-byte quad: the quads that hold the
+                // tile's columns are loaded aligned, made bytes, and the bytes
+                // shifted by the row's offset over the neighbouring lane's. (Four
+                // loads a quad, and a row a thread in the epilogue's loads and
+                // stores, at 1001 x 703, R = 9, two substeps: 28.7 -> 23.1 us.)
+#pragma unroll 1
+                for (int rg = warp - kEpiWarps; rg < kGroups; rg += kStageWarps) {
+                    const int row = rg * 8 + rl;
+                    const size_t at = size_t(wrap(y0 - g.r + row, H)) * W + size_t(x0 - P);
+                    const uint32_t shift = uint32_t(at) & 3u;
+                    const float4* quad = reinterpret_cast<const float4*>(src + (at - shift)) + (lane & 3);
+                    float4 a[NG + 1];
+#pragma unroll
+                    for (int f = 0; f < NG; ++f) a[f] = __ldg(quad + 4 * f);
+                    // The quad after the last granule's: the group's first lane reads it for the last.
+                    a[NG] = (lane & 3) == 0 && shift != 0u ? __ldg(quad + 4 * NG) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    uint32_t w[NG + 1][3];
+#pragma unroll
+                    for (int f = 0; f <= NG; ++f) {
+                        bad = bad || out_of_range(a[f]);
+                        pack_bytes(a[f], w[f]);
+                    }
+                    const int from = (lane & 3) == 3 ? lane - 3 : lane + 1;
+                    const uint32_t sel = 0x3210u + 0x1111u * shift;  // bytes shift .. shift + 3 of two words
+#pragma unroll
+                    for (int f = 0; f < NG; ++f)
+#pragma unroll
+                        for (int j = 0; j < 3; ++j) {
+                            const uint32_t next =
+                                __shfl_sync(0xffffffffu, (lane & 3) == 0 ? w[f + 1][j] : w[f][j], from);
+                            *reinterpret_cast<uint32_t*>(planes + uint32_t(j) * kPlane + (f * RA + row) * 16 + q) =
+                                __byte_perm(w[f][j], next, sel);
+                        }
+                }
+            } else {
 #pragma unroll 1
             for (int i0 = warp - kEpiWarps; i0 < kItems; i0 += kFlight * kStageWarps) {
                 float4 a[kFlight];
@@ -299,20 +353,14 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
                 for (int f = 0; f < kFlight; ++f) {
                     const int i = i0 + f * kStageWarps, gran = i / kGroups, row = (i - gran * kGroups) * 8 + rl;
-                    // 0 <= a < 2 exactly when the sign and the top exponent bit are
-                    // clear (-0 takes the FP32 form as well).
-                    bad = bad || (((__float_as_uint(a[f].x) | __float_as_uint(a[f].y)) |
-                                   (__float_as_uint(a[f].z) | __float_as_uint(a[f].w))) &
-                                  0xC0000000u) != 0u;
-                    const uint32_t v0 = __float2uint_rn(a[f].x * 8388608.0f), v1 = __float2uint_rn(a[f].y * 8388608.0f);
-                    const uint32_t v2 = __float2uint_rn(a[f].z * 8388608.0f), v3 = __float2uint_rn(a[f].w * 8388608.0f);
-                    const uint32_t l01 = __byte_perm(v0, v1, 0x5140), l23 = __byte_perm(v2, v3, 0x5140);
-                    const uint32_t h01 = __byte_perm(v0, v1, 0x7362), h23 = __byte_perm(v2, v3, 0x7362);
+                    bad = bad || out_of_range(a[f]);
+                    uint32_t w[3];
+                    pack_bytes(a[f], w);
                     unsigned char* o = planes + (gran * RA + row) * 16 + q;
-                    *reinterpret_cast<uint32_t*>(o) = __byte_perm(h01, h23, 0x5410);
-                    *reinterpret_cast<uint32_t*>(o + kPlane) = __byte_perm(l01, l23, 0x7632);
-                    *reinterpret_cast<uint32_t*>(o + 2 * kPlane) = __byte_perm(l01, l23, 0x5410);
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) *reinterpret_cast<uint32_t*>(o + uint32_t(j) * kPlane) = w[j];
                 }
+            }
             }
             if (bad) *reinterpret_cast<volatile int*>(&sh.bad[ai & 3u]) = int(ai) + 1;
             asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -405,21 +453,24 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int ty = tile / tiles_x, gx0 = (tile - ty * tiles_x) * kTX + kPart * half;
             const int gy = ty * kRows + 32 * quad + lane;
             // This thread's values of A, requested before the products are waited
-            // for (rows past the field read its last one).
-            const float* arow = src + size_t(min(gy, H - 1)) * W;
-            float4 av[kPart / 4];
+            // for (rows past the field read its last one). Rows that start
+            // anywhere in a quad are read two rows by 16 values an access and
+            // turned to one row a thread below.
+            const int gq = ty * kRows + 32 * quad;  // the warp's first row
+            float av[kPart];
             const bool whole = W % 4 == 0 && gx0 + kPart <= W;
+            if (whole) {
+                const float4* arow = reinterpret_cast<const float4*>(src + size_t(min(gy, H - 1)) * W + gx0);
 #pragma unroll
-            for (int c = 0; c < kPart / 4; ++c) {
-                if (whole) {
-                    av[c] = __ldg(reinterpret_cast<const float4*>(arow + gx0) + c);
-                } else {
-                    const int x = gx0 + 4 * c;
-                    av[c].x = x < W ? __ldg(arow + x) : 0.0f;
-                    av[c].y = x + 1 < W ? __ldg(arow + x + 1) : 0.0f;
-                    av[c].z = x + 2 < W ? __ldg(arow + x + 2) : 0.0f;
-                    av[c].w = x + 3 < W ? __ldg(arow + x + 3) : 0.0f;
+                for (int c = 0; c < kPart / 4; ++c) {
+                    const float4 a = __ldg(arow + c);
+                    av[4 * c] = a.x, av[4 * c + 1] = a.y, av[4 * c + 2] = a.z, av[4 * c + 3] = a.w;
                 }
+            } else {
+                const int x = gx0 + (lane & 15);
+#pragma unroll
+                for (int c = 0; c < kPart; ++c)
+                    av[c] = x < W ? __ldg(src + size_t(min(gq + 2 * c + (lane >> 4), H - 1)) * W + x) : 0.0f;
             }
             float2 sum[kPart / 2];  // growth sums of pixel pairs
 #pragma unroll 1
@@ -483,28 +534,47 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (lane == 0) bar_arrive(&sh.d_empty[db]);
             }
             if (!ok) break;  // its tile is left unwritten
-            if (gy >= H) continue;
-            float* orow = dst + size_t(gy) * W;
+            float* rows = reinterpret_cast<float*>(ring + kStages * kStage) + warp * (32 * kTurn);
+            float4* own = reinterpret_cast<float4*>(rows + lane * kTurn);
+            if (!whole) {
+#pragma unroll
+                for (int c = 0; c < kPart; ++c) rows[(2 * c + (lane >> 4)) * kTurn + (lane & 15)] = av[c];
+                __syncwarp();
+#pragma unroll
+                for (int c = 0; c < kPart / 4; ++c) {
+                    const float4 a = own[c];
+                    av[4 * c] = a.x, av[4 * c + 1] = a.y, av[4 * c + 2] = a.z, av[4 * c + 3] = a.w;
+                }
+                __syncwarp();
+            }
+            float4* orow = reinterpret_cast<float4*>(dst + size_t(min(gy, H - 1)) * W + gx0);
 #pragma unroll
             for (int c = 0; c < kPart; c += 8) {
-                const int gx = gx0 + c;
-                const float4 a = av[c / 4], b = av[c / 4 + 1];
-                float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+                float v[8];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    v[2 * j] = euler(v[2 * j], sum[c / 2 + j].x);
-                    v[2 * j + 1] = euler(v[2 * j + 1], sum[c / 2 + j].y);
+                    v[2 * j] = euler(av[c + 2 * j], sum[c / 2 + j].x);
+                    v[2 * j + 1] = euler(av[c + 2 * j + 1], sum[c / 2 + j].y);
                 }
-                noise_inject_clip(p, sh.ex, v, uint32_t(gx), uint32_t(gy));
-                if (whole) {
-                    float4* o = reinterpret_cast<float4*>(orow + gx);
-                    o[0] = make_float4(v[0], v[1], v[2], v[3]);
-                    o[1] = make_float4(v[4], v[5], v[6], v[7]);
-                } else {
+                noise_inject_clip(p, sh.ex, v, uint32_t(gx0 + c), uint32_t(gy));
+                const float4 lo = make_float4(v[0], v[1], v[2], v[3]), hi = make_float4(v[4], v[5], v[6], v[7]);
+                if (!whole) {
+                    own[c / 4] = lo;
+                    own[c / 4 + 1] = hi;
+                } else if (gy < H) {
+                    orow[c / 4] = lo;
+                    orow[c / 4 + 1] = hi;
+                }
+            }
+            if (!whole) {
+                const int x = gx0 + (lane & 15);
+                __syncwarp();
 #pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        if (gx + j < W) orow[gx + j] = v[j];
+                for (int c = 0; c < kPart; ++c) {
+                    const int r = 2 * c + (lane >> 4);
+                    if (gq + r < H && x < W) dst[size_t(gq + r) * W + x] = rows[r * kTurn + (lane & 15)];
                 }
+                __syncwarp();  // the rows are the next tile's
             }
         }
     }
@@ -530,7 +600,8 @@ template <int P>
 cudaError_t launch_t(int nk, const float* src, float* dst, const DirectTcPlan& plan, const float* weights,
                      const uint32_t* spans, const DirectGeometry& g, const StepParams& p, int* err, cudaStream_t s) {
     auto fn = direct_tc_kernel<P>;
-    constexpr size_t smem = 6 * size_t(kRows + 2 * P) * (kTX + 2 * P) + size_t(kStages) * kChunk * (1 + P / 16);
+    constexpr size_t smem = 6 * size_t(kRows + 2 * P) * (kTX + 2 * P) + size_t(kStages) * kChunk * (1 + P / 16) +
+                            sizeof(float) * kEpiWarps * 32 * kTurn;
     static fastfft::KernelState state;
     int per = 0;
     cudaError_t e = fastfft::prepare(state, fn, kThreads, smem, per);
@@ -618,29 +689,38 @@ bool direct_tc_tables(const std::vector<std::vector<float>>& luts, int r, Direct
 
 // Frame times in us as measured back to back on a B200 (148 SMs), one kernel:
 //                      R = 3        5        9        13       20       32
-//   128 x 128   FP32    7.1      9.1      9.1      11.2     13.3     21.7
-//               bytes   9.4     10.0     11.4      12.6     20.0     26.7
-//   512 x 512   FP32    9.1     11.2     15.3      19.4     29.7     62.4
-//               bytes   9.7     10.3     11.6      13.1     20.7     27.2
-//   1280 x 720  FP32   13.3     19.5     31.9      48.1     84.3    197.6
-//               bytes  13.4     14.2     15.8      18.4     30.2     44.1
-//   1920 x 1080 FP32   19.4     30.4     55.6      76.7    150.7    345.8
-//               bytes  21.1     22.8     27.1      32.3     47.4     74.8
+//   128 x 128   FP32    7.3      8.4      9.1      10.5     13.1     20.9
+//               bytes   9.9     10.5     11.9      13.2     20.7     27.4
+//   512 x 512   FP32    9.0     10.4     13.2      17.3     27.5     62.1
+//               bytes  10.1     10.9     12.1      13.5     21.2     27.8
+//   1001 x 703  FP32   11.1     14.7     25.1      37.2     63.4    133.6
+//               bytes  15.1     15.8     18.5      20.8     32.1     46.3
+//   1280 x 720  FP32   11.3     17.2     29.6      43.9     78.7    183.8
+//               bytes  14.3     14.8     16.1      19.0     30.7     44.8
+//   1920 x 1080 FP32   17.3     25.5     46.0      72.1    134.1    314.5
+//               bytes  21.1     21.8     25.5      29.5     48.1     75.7
 // (before the byte form the FP32 column was 205 us at 1280 x 720, R = 32 and 81
 // at 1920 x 1080, R = 13). Both sides are modelled from them: the byte form by
 // its fixed 8.5 us (launch, first tile's staging, last epilogue) and, per round
 // of tiles over the SMs, the larger of the products (87 ns a chunk) and the
 // staging and epilogue (3.4 us); the FP32 form by its 8-tap multiply-adds (3.7e-8
 // us each on fields that fill the SMs evenly, 4.8e-8 below) and 5e-6 us a
-// pixel. Kernels of few taps stay on the FP32 form, whose rounding grows with
+// pixel. A CTA of the byte form holds its SM's tensor memory, so kernels of other
+// contexts fill only the SMs it leaves free; the time a frame costs beside
+// others (its share of the SMs, three quarters of it overlapped at best) counts
+// as much as its own, and its own is at most a tenth longer. Two substeps of 1001 x 703 with noise, jitter and
+// blobs, FP32 / bytes: R = 5 alone 35.2 / 39.2, three contexts 18.9 / 26.3 us;
+// R = 9 57.4 / 45.3 and 34.0 / 30.4 us. Kernels of few taps stay on the FP32 form, whose rounding grows with
 // the taps while the byte form's is fixed (they cross at R = 4, 49 taps).
 bool direct_tc_faster(const DirectTcTables& t, uint64_t fp32_taps, int w, int h, int sms) {
     if (t.min_taps < 60) return false;
     const double px = double(w) * h;
     const int tiles = ((w + kTX - 1) / kTX) * ((h + kRows - 1) / kRows), rounds = (tiles + sms - 1) / std::max(1, sms);
     const double bytes = 8.5 + rounds * std::max(0.087 * t.chunks, 3.4);
+    const double share = 0.75 * bytes * std::min(1.0, double(tiles) / std::max(1, sms));
+    const double work = px * (double(fp32_taps) * 3.7e-8 + 5e-6);  // of the FP32 form, the SMs full
     const double fp32 = 7.0 + px * (double(fp32_taps) * (px < 1.5e6 ? 4.8e-8 : 3.7e-8) + 5e-6);
-    return bytes < fp32;
+    return bytes + share < fp32 + work && bytes < 1.1 * fp32;
 }
 
 cudaError_t launch_direct_tc(int nk, const float* src, float* dst, const DirectTcPlan& plan, const float* weights,
