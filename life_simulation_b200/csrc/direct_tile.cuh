@@ -17,8 +17,8 @@ namespace {
 
 constexpr int PX = 8;  // taps per chunk along x (and the default outputs per thread)
 
-// OX outputs per thread along x: 8, or 16 on large tiles (half the input
-// loads per multiply-add); OY output rows per thread: 1, or 2 on large tiles
+// OX outputs per thread along x: 8, 16 on large tiles (half the input loads per
+// multiply-add), or 4 for a batch of few tiles (launch_direct_worlds); OY output rows per thread: 1, or 2 on large tiles
 // (each staged input row chunk then feeds two kernel rows: half the input
 // loads again). Each output's sum runs in the same order in every variant,
 // so they all give the same bits.

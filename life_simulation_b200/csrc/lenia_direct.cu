@@ -23,12 +23,14 @@
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdint>
 #include <cstring>
 #include <mutex>
 
 #include "direct_tile.cuh"
+#include "fft_fast_common.cuh"
 #include "lenia_device.cuh"
 #include "lenia_kernels.h"
 
@@ -51,14 +53,14 @@ __global__ void __launch_bounds__(DirectTile<TW, TH, OX, OY>::kThreads * S)
 // Many worlds in one launch: CTA i computes tile tiles[i] = (world, tile x,
 // tile y) of that world; each world brings its own state buffers, LUT,
 // geometry and growth parameters.
-template <int TW, int TH>
-__global__ void __launch_bounds__(DirectTile<TW, TH>::kThreads)
+template <int TW, int TH, int OX>
+__global__ void __launch_bounds__(DirectTile<TW, TH, OX>::kThreads)
     direct_worlds_kernel(const DirectWorld* __restrict__ worlds, const int3* __restrict__ tiles) {
     __shared__ DirectWorld w;
     const int3 t = tiles[blockIdx.x];
     if (threadIdx.x == 0) w = worlds[t.x];
     __syncthreads();
-    direct_tile<TW, TH, 1, 1, PX, 1, true>(w.src, w.dst, w.weights, w.spans, w.g, w.p, t.y * TW, t.z * TH, nullptr, nullptr);
+    direct_tile<TW, TH, 1, 1, OX, 1, true>(w.src, w.dst, w.weights, w.spans, w.g, w.p, t.y * TW, t.z * TH, nullptr, nullptr);
 }
 
 template <int TW, int TH, int NK, int S, int OX, int OY>
@@ -212,17 +214,32 @@ cudaError_t launch_direct_worlds(const DirectWorld* worlds, const int3* tiles, i
     // 128 x 128 R = 8 1022 / 600 us, 512 x 512 R = 12 1594 / 1116 us; 48 worlds
     // 512 x 512 R = 12 29965 / 23156 us.
     constexpr int TW = 32, TH = 16;
-    DirectGeometry g;
-    g.r = max_r;
-    g.ksize = 2 * max_r + 1;
-    g.xp = (max_r + 3) / 4 * 4;
-    g.wp = 2 * g.xp + 8;
-    const size_t smem = direct_smem_bytes(kDirectTile32x16, 1, g);
-    auto fn = direct_worlds_kernel<TW, TH>;
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    const auto bytes = [](int r) {
+        DirectGeometry g;
+        g.r = r;
+        g.ksize = 2 * r + 1;
+        g.xp = (r + 3) / 4 * 4;
+        g.wp = 2 * g.xp + 8;
+        return direct_smem_bytes(kDirectTile32x16, 1, g);
+    };
+    const size_t smem = bytes(max_r);
+    // Up to six tiles an SM a tile's own time is what the launch takes: a chain
+    // of taps per thread, shorter with four outputs a thread (128 threads) than
+    // with eight, whose half as many loads per multiply-add pay when the SMs are
+    // full. 60 substeps, eight / four outputs: one world 128 x 128 R = 12 859 /
+    // 691 us, 512 x 512 R = 12 (512 tiles) 1116 / 1031; 8 worlds of four sizes, 5
+    // of them direct 4158 / 3181; 48 worlds 128 x 128 R = 12 (1536 tiles) 1985 /
+    // 2264. Each output's sum runs in the same order either way: the same bits.
+    const bool few = ntiles <= 6 * fastfft::sms();
+    auto fn = few ? direct_worlds_kernel<TW, TH, 4> : direct_worlds_kernel<TW, TH, PX>;
+    const int threads = few ? DirectTile<TW, TH, 4>::kThreads : DirectTile<TW, TH>::kThreads;
+    // The limit of the largest radius: a batch of smaller ones must not lower
+    // another's between its capture and its replays.
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         int(std::max(smem, bytes(kMaxRadius))));
     if (e != cudaSuccess) return e;
     if (ntiles <= 0) return cudaSuccess;
-    fn<<<ntiles, DirectTile<TW, TH>::kThreads, smem, stream>>>(worlds, tiles);
+    fn<<<ntiles, threads, smem, stream>>>(worlds, tiles);
     return cudaGetLastError();
 }
 

@@ -704,14 +704,15 @@ bool direct_tc_tables(const std::vector<std::vector<float>>& luts, int r, Direct
 // its fixed 8.5 us (launch, first tile's staging, last epilogue) and, per round
 // of tiles over the SMs, the larger of the products (87 ns a chunk) and the
 // staging and epilogue (3.4 us); the FP32 form by its 8-tap multiply-adds (3.7e-8
-// us each on fields that fill the SMs evenly, 4.8e-8 below) and 5e-6 us a
-// pixel. A CTA of the byte form holds its SM's tensor memory, so kernels of other
-// contexts fill only the SMs it leaves free; the time a frame costs beside
+// us each on fields that fill the SMs evenly, 4.8e-8 below) and 5e-6 us a pixel.
+// A CTA of the byte form holds its SM's tensor memory, so kernels of other
+// contexts fill only the SMs it leaves free: the time a frame costs beside
 // others (its share of the SMs, three quarters of it overlapped at best) counts
-// as much as its own, and its own is at most a tenth longer. Two substeps of 1001 x 703 with noise, jitter and
-// blobs, FP32 / bytes: R = 5 alone 35.2 / 39.2, three contexts 18.9 / 26.3 us;
-// R = 9 57.4 / 45.3 and 34.0 / 30.4 us. Kernels of few taps stay on the FP32 form, whose rounding grows with
-// the taps while the byte form's is fixed (they cross at R = 4, 49 taps).
+// as much as its own, and its own is at most a tenth longer. Two substeps of
+// 1001 x 703 with noise, jitter and blobs, FP32 / bytes: R = 5 alone 35.2 / 39.2
+// us, beside two others 18.9 / 26.3; R = 9 57.4 / 45.3 and 34.0 / 30.4 us.
+// Kernels of few taps stay on the FP32 form, whose rounding grows with the taps
+// while the byte form's is fixed (they cross at R = 4, 49 taps).
 bool direct_tc_faster(const DirectTcTables& t, uint64_t fp32_taps, int w, int h, int sms) {
     if (t.min_taps < 60) return false;
     const double px = double(w) * h;

@@ -42,3 +42,21 @@ def test_small_fields_against_fp64_oracle(monkeypatch, w, h):
     # 81 taps, each rounded once, times the growth's slope dt * 1.22 / sigma.
     assert np.abs(m.field() - o.encode(0, 1)).max() <= 81 * 2.0**-24 * 8.1 + 2e-7
     m.close()
+
+
+@pytest.mark.parametrize("few", [1, 40])
+def test_batch_tiles_of_four_and_eight_outputs_agree(few):
+    """`few` worlds of 64 tiles each, below and above the launch's line of tiles
+    per SM: the same world in either batch is the same bits."""
+    a = np.random.default_rng(7).random((256, 128), np.float32)
+    out = []
+    for n in (1, few):
+        b = lb.LeniaBatch([lb.make_world(width=128, height=256, radius=9, mu=0.15, sigma=0.03, dt=0.1, seed=5)] * n,
+                          lb.BATCH_DIRECT)
+        for i in range(n):
+            b.upload(i, a)
+        b.step(3)
+        out += [b.field(i) for i in range(n)]
+        b.close()
+    for f in out[1:]:
+        np.testing.assert_array_equal(f, out[0])
