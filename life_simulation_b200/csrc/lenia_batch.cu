@@ -661,12 +661,14 @@ int lenia_batch_create(const lenia_world* worlds, uint32_t n, uint32_t policy, l
         // Policy AUTO: the path whose launches, each on its own, cost a world
         // less -- the spectral step of its size class, shared by the class's
         // worlds, against its share by pixel-taps of the direct launch over
-        // every world that has both paths. The three constants are fitted to
-        // what timing those launches at creation picked (3456 worlds in
-        // batches of 1 to 60: 97 % the same; timing disagreed with itself on
-        // 1 % between two processes): 6 us a class's two spectral launches,
-        // 40 fs a pixel-tap of a full direct launch, and a direct launch no
-        // shorter than 19 us and 6.3 ns per tap of its largest kernel.
+        // every world that has both paths. The constants are fitted to what
+        // timing those launches at creation picked (3456 worlds of mixed radii
+        // in batches of 1 to 60: 97 % the same, and 95 % of 1320 batches of one
+        // size and radius; timing disagreed with itself on 1 % between two
+        // processes): 4.74 us a class's two spectral launches, 31.3 fs a
+        // pixel-tap of a full direct launch, and a direct launch no shorter than
+        // 0.52 us and 0.96 us per pixel of its largest radius (a tile's halo and
+        // its threads' chain of taps).
         // A rule instead of the timing gives a batch the same paths, and so the
         // same bits, every time. It deliberately keeps the line where the timing
         // had it, since such fields amplify the two paths' rounding (2e-4 after
@@ -675,16 +677,16 @@ int lenia_batch_create(const lenia_world* worlds, uint32_t n, uint32_t policy, l
         // (4 worlds x 60 substeps 1.1 against 1.6 to 1.8 ms, 8 worlds 1.2 against
         // 1.7 to 2.4; from 48 worlds on they are level).
         if (policy == LENIA_BATCH_AUTO) {
-            constexpr double kClass = 6e-6, kTap = 40e-15, kDirect = 19e-6, kLargest = 6.3e-9;
+            constexpr double kClass = 4.74e-6, kTap = 31.3e-15, kDirect = 0.52e-6, kRadius = 0.961e-6;
             const auto taps = [&](uint32_t i) { return double(worlds[i].width) * worlds[i].height * nnz[i]; };
             double total = 0.0;
             uint32_t largest = 0;
             for (uint32_t i = 0; i < n; ++i)
                 if (can_direct[i] && can_fft[i]) {
                     total += taps(i);
-                    largest = std::max(largest, nnz[i]);
+                    largest = std::max(largest, worlds[i].radius);
                 }
-            const double per_tap = total > 0.0 ? std::max(kTap, (kDirect + kLargest * largest) / total) : kTap;
+            const double per_tap = total > 0.0 ? std::max(kTap, (kDirect + kRadius * largest) / total) : kTap;
             for (uint32_t i = 0; i < n; ++i)
                 if (can_direct[i] && can_fft[i])
                     b.path[i] = taps(i) * per_tap <= kClass / double(class_members[size_t(cls[i])].size()) ? LENIA_CONV_DIRECT
