@@ -30,14 +30,16 @@
 // What bounds it: the operands' shared-memory reads. A product of N columns
 // takes max(46, 32 + N / 4) cycles (measured, N <= 128: 4 KB of X and 32 N
 // bytes of T at 128 bytes a cycle, against N / 2 cycles of math), so small N
-// is lost; the levels of a chunk are side by side in D and T's byte planes in
-// [w0 | w1 | w2] rows, which makes the eight byte products three: X0 against
-// all of T (N = 96) into levels 0..2, X1 likewise into levels 1..3, X2 against
-// [w0 | w1] (N = 64) into levels 2 and 3: 161 cycles a chunk, where eight
-// products of N = 32 took 366. Wider tiles read X less often but clip T's
-// window, and came out behind. The T blocks (3 KB a chunk) come through a ring of bulk copies from
-// L2, requested by one warp and multiplied by another, whose loop is uniform
-// over the warp.
+// is lost; T's byte planes are side by side in [w0 | w1 | w2] rows, which makes
+// the eight byte products three: X0 against all of T (N = 96), X1 likewise, X2
+// against [w0 | w1] (N = 64): 160 cycles a chunk, where eight products of N =
+// 32 took 366. Each of the three adds into accumulator columns of its own
+// (levels 0..2, 1..3 and 2..3), summed in the epilogue: tcgen05.mma orders
+// successive products only where accumulator and shape are the same, so windows
+// of different products may not overlap. Wider tiles read X less often but clip
+// T's window, and came out behind. The T blocks (3 KB a chunk) come through a
+// ring of bulk copies from L2, requested by one warp and multiplied by another,
+// whose loop is uniform over the warp.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -57,15 +59,17 @@ constexpr int kRows = 128;             // output rows of a tile (accumulator lan
 constexpr int kTX = 32;                // output columns of a tile
 constexpr int kPart = kTX / 2;         // output columns per epilogue thread
 // Warps: 0..7 epilogue (tensor-memory lane quadrant warp % 4, half of the
-// columns warp / 4), 8..15 stage the halo tiles, 16 and 17 issue the products
-// (a product is issued when the one before it in its warp has been read, so
-// one warp's waits leave the tensor cores idle; two warps on alternate T
-// blocks, each with its own accumulator, fill each other's), 18 requests the
-// T blocks.
-constexpr int kEpiWarps = 8, kStageWarps = 8, kMmaWarp = 16, kMmaWarps = 2, kLoadWarp = 18;
-constexpr int kThreads = 32 * 19;
+// columns warp / 4), 8..15 stage the halo tiles, then kMmaWarps that issue the
+// products of alternate T blocks into accumulators of their own, and one that
+// requests the T blocks.
+constexpr int kEpiWarps = 8, kStageWarps = 8, kMmaWarp = 16, kMmaWarps = 2, kLoadWarp = kMmaWarp + kMmaWarps;
+constexpr int kThreads = 32 * (kLoadWarp + 1);
 constexpr int kStages = 6;             // T blocks in flight
-constexpr uint32_t kCols = 512;        // tensor-memory columns: per buffer and issuing warp 128 (four levels)
+// Tensor-memory columns of one issuing warp's accumulators: X0's levels 0..2
+// from column 0, X1's 1..3 from 96, X2's 2..3 from 192. Sets: kMmaWarps for each
+// of kBufs tiles (or kernels) in flight.
+constexpr uint32_t kCols = 512, kAccX1 = 3 * kTX, kAccX2 = 6 * kTX, kAccCols = 8 * kTX;
+constexpr uint32_t kBufs = kCols / (kAccCols * kMmaWarps);
 constexpr uint32_t kChunk = 96u * 32u; // bytes of one chunk's T: 96 rows of 32 k
 constexpr int kTurn = kPart + 4;       // pitch (floats) of the rows an epilogue warp turns A and A' in
 constexpr uint32_t kPolls = 1u << 20;  // polls of a barrier before a CTA gives up (about a second)
@@ -85,6 +89,12 @@ constexpr uint32_t idesc(uint32_t n) {
     return (2u << 4) | (0u << 7) | (1u << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24);
 }
 
+// 1 in one lane of a converged warp: the one that issues (and so commits) its products.
+__device__ __forceinline__ uint32_t elected() {
+    uint32_t lead;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(lead));
+    return lead;
+}
 // Issued by the one lane whose `lead` is set, in a converged warp: a
 // predicate on the instruction, not a branch around it, so that the loop
 // that computes the descriptors stays uniform and keeps them in uniform
@@ -107,15 +117,17 @@ __device__ __forceinline__ void commit(uint64_t* bar, uint32_t lead) {
 }
 // The products of one kernel row: NQ + 1 chunks from operand addresses a, b;
 // PLANE: bytes of a byte plane, STEP: bytes of two granules (a chunk's 32
-// columns).
+// columns). acc = 0: the first products of a kernel, which set all of the three
+// accumulators' columns.
 template <int NQ, uint32_t PLANE, uint32_t STEP>
 __device__ __forceinline__ void mma_row(uint32_t tmem, uint32_t a, uint32_t b, uint32_t acc, uint32_t lead) {
 #pragma unroll
     for (int c = 0; c <= NQ; ++c) {
         const uint32_t ac = a + uint32_t(c) * (STEP / 16), bc = b + uint32_t(c) * (kChunk / 16);
-        mma_i8(tmem, ac, bc, idesc(96), c > 0 ? 1u : acc, lead);
-        mma_i8(tmem + kTX, ac + PLANE / 16, bc, idesc(96), 1, lead);
-        mma_i8(tmem + 2 * kTX, ac + 2 * (PLANE / 16), bc, idesc(64), 1, lead);
+        const uint32_t add = c > 0 ? 1u : acc;
+        mma_i8(tmem, ac, bc, idesc(96), add, lead);
+        mma_i8(tmem + kAccX1, ac + PLANE / 16, bc, idesc(96), add, lead);
+        mma_i8(tmem + kAccX2, ac + 2 * (PLANE / 16), bc, idesc(64), add, lead);
     }
 }
 __device__ __forceinline__ void bar_init(uint64_t* bar, uint32_t count) {
@@ -159,15 +171,12 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
 
-// 8 consecutive accumulator columns of this warp's lane quadrant (not
+// 4 consecutive accumulator columns of this warp's lane quadrant (not
 // waited for).
-__device__ __forceinline__ void tmem_ld8(uint32_t addr, int32_t (&v)[8]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+__device__ __forceinline__ void tmem_ld4(uint32_t addr, int32_t (&v)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
                  : "r"(addr));
-}
-__device__ __forceinline__ void tmem_zero8(uint32_t addr) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1};\n" ::"r"(addr), "r"(0) : "memory");
 }
 
 __device__ __forceinline__ int wrap(int v, int n) {
@@ -213,8 +222,8 @@ __device__ __noinline__ float direct_point(const float* __restrict__ src, const 
 struct TcShared {
     uint64_t t_full[kStages], t_empty[kStages];  // T blocks
     uint64_t a_full[2], a_empty[2];              // staged halo tiles
-    uint64_t d_full[2], d_empty[2];              // accumulators
-    uint64_t drain[kMmaWarps];                              // products in flight when a wait ran out
+    uint64_t d_full[kBufs], d_empty[kBufs];      // accumulators
+    uint64_t drain[kMmaWarps];                   // products in flight when a wait ran out
     int bad[4];     // tile count + 1 of the last tile of slot (count % 4) with a value outside the byte form
     int stop;       // a wait ran out
     uint32_t tmem;  // tensor-memory address
@@ -224,7 +233,7 @@ struct TcShared {
 // P: halo columns each side (16 for r <= 16, else 32); the staged planes have
 // 128 + 2 P rows, of which 128 + 2 r are read. One CTA per SM loops
 // over tiles; staging, products and epilogue of successive tiles overlap (two
-// staged tiles, two accumulators).
+// staged tiles, kBufs sets of accumulators).
 template <int P>
 __global__ void __launch_bounds__(kThreads, 1)
     direct_tc_kernel(const float* __restrict__ src, float* __restrict__ dst, const __grid_constant__ DirectTcPlan plan,
@@ -249,6 +258,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int i = 0; i < 2; ++i) {
             bar_init(&sh.a_full[i], kStageWarps);
             bar_init(&sh.a_empty[i], kMmaWarps);
+        }
+        for (uint32_t i = 0; i < kBufs; ++i) {
             bar_init(&sh.d_full[i], kMmaWarps);
             bar_init(&sh.d_empty[i], kEpiWarps);
         }
@@ -267,18 +278,6 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, sh.tmem, 0);
-    // Level 3 starts at zero (the first product of a kernel sets levels 0 to
-    // 2); from then on the epilogue clears it as it reads it.
-    if (warp < kEpiWarps) {
-        const uint32_t at = tmem + (uint32_t(32 * (warp & 3)) << 16) + uint32_t(3 * kTX + kPart * (warp >> 2));
-#pragma unroll
-        for (int c = 0; c < kPart; c += 8)
-#pragma unroll
-            for (uint32_t d = 0; d < kCols; d += 128) tmem_zero8(at + d + uint32_t(c));
-        asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
-        fence_before();
-    }
-    __syncthreads();
 
     if (warp >= kEpiWarps && warp < kEpiWarps + kStageWarps) {
         // ---- Stage the halo tiles as three byte planes, [16-column granule]
@@ -389,10 +388,9 @@ __global__ void __launch_bounds__(kThreads, 1)
                 bar_wait_slow(&sh.t_full[i % kStages], (i / kStages) & 1u, &never);
         }
     } else if (warp >= kMmaWarp && warp < kMmaWarp + kMmaWarps) {
-        // ---- Products of every second T block.
+        // ---- Products of every kMmaWarps-th T block.
         const int m = warp - kMmaWarp;
-        uint32_t lead;
-        asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(lead));
+        const uint32_t lead = elected();
         const uint32_t b_base = desc_lo(smem_u32(ring), kChunk / 2);
         uint32_t ai = 0, di = 0, st = 0, ph = 0;  // ring stage and its phase
         bool ok = true;
@@ -402,14 +400,14 @@ __global__ void __launch_bounds__(kThreads, 1)
             ok = bar_wait(&sh.a_full[buf], (ai >> 1) & 1u, &sh.stop);
 #pragma unroll 1
             for (int k = 0; k < nk && ok; ++k, ++di) {
-                const uint32_t db = di & 1u, d = tmem + db * 256u + uint32_t(m) * 128u;
-                if (di >= 2) ok = bar_wait(&sh.d_empty[db], ((di >> 1) - 1u) & 1u, &sh.stop);
+                const uint32_t db = di % kBufs, d = tmem + (db * kMmaWarps + uint32_t(m)) * kAccCols;
+                if (di >= kBufs) ok = bar_wait(&sh.d_empty[db], (di / kBufs - 1u) & 1u, &sh.stop);
                 fence_after();
-                uint32_t acc = 0;  // the first product of N = 96 sets the accumulator
+                uint32_t acc = 0;  // the first products set the accumulators
                 const int r0 = plan.first[k], r1 = plan.first[k + 1];
 #pragma unroll 1
                 for (int r = r0; r < r1 && ok; ++r) {
-                    if (((r - r0) & 1) == m) {
+                    if ((r - r0) % kMmaWarps == m) {
                         const uint32_t row = plan.rows[r], nq = row >> 14;
                         const uint32_t a = a_base - nq * uint32_t(RA), b = b_base + st * (kStage / 16);
                         const uint32_t dy0 = row & 127u, dy1 = (row >> 7) & 127u;
@@ -475,63 +473,70 @@ __global__ void __launch_bounds__(kThreads, 1)
             float2 sum[kPart / 2];  // growth sums of pixel pairs
 #pragma unroll 1
             for (int k = 0; k < nk; ++k, ++di) {
-                const uint32_t db = di & 1u;
-                if (!(ok = bar_wait(&sh.d_full[db], (di >> 1) & 1u, &sh.stop))) break;
+                const uint32_t db = di % kBufs;
+                if (!(ok = bar_wait(&sh.d_full[db], (di / kBufs) & 1u, &sh.stop))) break;
                 fence_after();
                 const bool bytes = *reinterpret_cast<volatile int*>(&sh.bad[ai & 3u]) != int(ai) + 1;
                 const float scale = pick(plan.scale, k);
                 const float s0 = scale * 512.0f, s1 = scale * 2.0f;
                 const GrowthPair gp(pick(p.mu, k), 1.0f / pick(p.sigma, k), pick(p.weight, k), euler.asym);
-                const bool two = plan.first[k + 1] - plan.first[k] > 1;  // T blocks for the second issuing warp
+                // T blocks of kernel k: the issuing warps that had one.
+                const int blocks = plan.first[k + 1] - plan.first[k];
+                float u[kPart];
 #pragma unroll
-                for (int c = 0; c < kPart; c += 8) {
-                    float u[8];
-                    int32_t l0[8], l1[8], l2[8], l3[8], m0[8] = {}, m1[8] = {}, m2[8] = {}, m3[8] = {};
-                    const uint32_t d = mine + db * 256u + uint32_t(c);
-                    tmem_ld8(d, l0);
-                    tmem_ld8(d + kTX, l1);
-                    tmem_ld8(d + 2 * kTX, l2);
-                    tmem_ld8(d + 3 * kTX, l3);
-                    if (two) {
-                        tmem_ld8(d + 128, m0);
-                        tmem_ld8(d + 128 + kTX, m1);
-                        tmem_ld8(d + 128 + 2 * kTX, m2);
-                        tmem_ld8(d + 128 + 3 * kTX, m3);
-                    }
-                    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-                    tmem_zero8(d + 3 * kTX);
-                    tmem_zero8(d + 128 + 3 * kTX);
-                    // Levels 2 and 3 join level 1 as integers (rounded at 2^-31 of the sum).
+                for (int c = 0; c < kPart; c += 4) {
+                    int32_t l0[4] = {}, l1[4] = {}, l2[4] = {}, l3[4] = {};
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const int32_t v2 = l2[j] + m2[j] + ((l3[j] + m3[j] + 128) >> 8);
-                        const int32_t v1 = l1[j] + m1[j] + ((v2 + 128) >> 8);
-                        u[j] = fmaf(float(l0[j] + m0[j]), s0, float(v1) * s1);
-                    }
-                    if (!bytes) {
-#pragma unroll 1
-                        for (int j = 0; j < 8; ++j) {
-                            const float v = gy < H && gx0 + c + j < W
-                                                ? direct_point(src, weights, spans, g, W, H, k, gx0 + c + j, gy)
-                                                : 0.0f;
+                    for (int m = 0; m < kMmaWarps; ++m) {
+                        if (m >= blocks) break;
+                        const uint32_t d = mine + (db * kMmaWarps + uint32_t(m)) * kAccCols + uint32_t(c);
+                        int32_t x00[4], x01[4], x02[4], x11[4], x12[4], x13[4], x22[4], x23[4];  // X's byte, level
+                        tmem_ld4(d, x00);
+                        tmem_ld4(d + kTX, x01);
+                        tmem_ld4(d + 2 * kTX, x02);
+                        tmem_ld4(d + kAccX1, x11);
+                        tmem_ld4(d + kAccX1 + kTX, x12);
+                        tmem_ld4(d + kAccX1 + 2 * kTX, x13);
+                        tmem_ld4(d + kAccX2, x22);
+                        tmem_ld4(d + kAccX2 + kTX, x23);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
-                            for (int i = 0; i < 8; ++i) u[i] = i == j ? v : u[i];
+                        for (int j = 0; j < 4; ++j) {
+                            l0[j] += x00[j];
+                            l1[j] += x01[j] + x11[j];
+                            l2[j] += x02[j] + x12[j] + x22[j];
+                            l3[j] += x13[j] + x23[j];
                         }
                     }
+                    // Levels 2 and 3 join level 1 as integers (rounded at 2^-31 of the sum).
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
-                        const float2 uu = make_float2(u[2 * j], u[2 * j + 1]);
-                        const float2 t =
-                            gp.term_near(uu, jitter ? mu_jitter_pair(p, sh.ex, uint32_t(gx0 + c + 2 * j), uint32_t(gy))
-                                                    : make_float2(0.0f, 0.0f));
-                        float2& to = sum[c / 2 + j];
-                        to = k == 0 ? t : __fadd2_rn(to, t);
+                        const int32_t v2 = l2[j] + ((l3[j] + 128) >> 8);
+                        const int32_t v1 = l1[j] + ((v2 + 128) >> 8);
+                        u[c + j] = fmaf(float(l0[j]), s0, float(v1) * s1);
                     }
                 }
-                asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
                 fence_before();
                 __syncwarp();
                 if (lane == 0) bar_arrive(&sh.d_empty[db]);
+                if (!bytes) {
+#pragma unroll 1
+                    for (int j = 0; j < kPart; ++j) {
+                        const float v = gy < H && gx0 + j < W
+                                            ? direct_point(src, weights, spans, g, W, H, k, gx0 + j, gy)
+                                            : 0.0f;
+#pragma unroll
+                        for (int i = 0; i < kPart; ++i) u[i] = i == j ? v : u[i];
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < kPart / 2; ++j) {
+                    const float2 uu = make_float2(u[2 * j], u[2 * j + 1]);
+                    const float2 t =
+                        gp.term_near(uu, jitter ? mu_jitter_pair(p, sh.ex, uint32_t(gx0 + 2 * j), uint32_t(gy))
+                                                : make_float2(0.0f, 0.0f));
+                    sum[j] = k == 0 ? t : __fadd2_rn(sum[j], t);
+                }
             }
             if (!ok) break;  // its tile is left unwritten
             float* rows = reinterpret_cast<float*>(ring + kStages * kStage) + warp * (32 * kTurn);
@@ -586,7 +591,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (warp >= kMmaWarp && warp < kMmaWarp + kMmaWarps) {
             int never = 0;
             fence_after();
-            commit(&sh.drain[warp - kMmaWarp], lane == 0 ? 1u : 0u);
+            commit(&sh.drain[warp - kMmaWarp], elected());
             bar_wait_slow(&sh.drain[warp - kMmaWarp], 0, &never);
         }
         __syncthreads();
