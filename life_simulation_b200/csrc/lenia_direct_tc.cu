@@ -4,16 +4,24 @@
 // epilogue: the same update as lenia_direct.cu (the work of leniaStep,
 // Shaders/Field/Lenia.metal:63-128, for up to 4 kernel tables).
 //
-// Arithmetic. A field value a in [0, 2) is the 24-bit fixed-point number
-// A = rint(a 2^23) = a0 2^16 + a1 2^8 + a2 (unsigned bytes), a weight w the
-// number rint(w 2^e) = w0 2^16 + w1 2^8 + w2 (signed bytes; e the largest
+// Arithmetic. A field value a in [0, 2) is the 32-bit fixed-point number
+// A = rint(a 2^31) = a0 2^24 + a1 2^16 + a2 2^8 + a3 (unsigned bytes), a weight
+// w the number rint(w 2^e) = w0 2^16 + w1 2^8 + w2 (signed bytes; e the largest
 // exponent that keeps the table in range). The products of byte i and byte j
-// go to the integer sum of level i + j; levels 0 to 3 (all but the last of the
-// nine products) are summed exactly -- 3 * 4225 taps * 255 * 128 < 2^31 -- and
+// go to the integer sum of level i + j; levels 0 to 3 (nine of the twelve
+// products) are summed exactly -- 3 * 4225 taps * 255 * 128 < 2^31 -- and
 // combined in FP32 once: U = L0 2^(9-e) + (L1 + L2 / 2^8 + L3 / 2^16) 2^(1-e).
-// What is dropped is 2^-32 of a tap's share, so the sum's error is the
-// rounding of that last combination, where the FP32 form rounds once per tap;
-// and an integer sum is the same in any order. A tile whose halo holds a value outside [0, 2)
+//
+// Its error: a value of 2^-8 or more is exact, a fainter one off by up to 2^-32;
+// the weights' rounding, half a unit of 2^-e a tap, is carried from tap to tap so
+// that it cancels where the field is smooth; the levels left out weigh 2^-32 of
+// a tap's share; the last combination rounds three times (two conversions, one
+// FMA). The FP32 form rounds once per tap. U enters the growth as U - mu, which FP32
+// rounds at 2^-25 |mu| or more away from mu, so that 2^-32 stays below the FP32
+// form's own rounding for |mu| >= 2^-6, and kernels nearer zero run on the FP32
+// form (direct_tc_holds). With 24-bit values, rint(a 2^23), a field of 1e-3
+// had a potential off by 6e-5 of itself, two orders above the FP32 form's.
+// An integer sum is the same in any order. A tile whose halo holds a value outside [0, 2)
 // (an uploaded field may: infinities, NaN, negative values) takes the FP32
 // loop below, tap by tap in the order of lenia_direct.cu.
 //
@@ -30,14 +38,15 @@
 // What bounds it: the operands' shared-memory reads. A product of N columns
 // takes max(46, 32 + N / 4) cycles (measured, N <= 128: 4 KB of X and 32 N
 // bytes of T at 128 bytes a cycle, against N / 2 cycles of math), so small N
-// is lost; T's byte planes are side by side in [w0 | w1 | w2] rows, which makes
-// the eight byte products three: X0 against all of T (N = 96), X1 likewise, X2
-// against [w0 | w1] (N = 64): 160 cycles a chunk, where eight products of N =
-// 32 took 366. Each of the three adds into accumulator columns of its own
-// (levels 0..2, 1..3 and 2..3), summed in the epilogue: tcgen05.mma orders
-// successive products only where accumulator and shape are the same, so windows
-// of different products may not overlap. Wider tiles read X less often but clip
-// T's window, and came out behind. The T blocks (3 KB a chunk) come through a
+// is lost; T's byte planes are side by side in [0 | w0 | w1 | w2] rows, which makes
+// the nine byte products four: X0 against [w0 | w1 | w2] (N = 96), X1 likewise,
+// X2 against [w0 | w1] (N = 64), X3 against [0 | w0] (N = 64): 208 cycles a
+// chunk, where nine products of N = 32 would take 414. X0, X1 and the pair X2,
+// X3 add into accumulator columns of their own (levels 0..2, 1..3 and 2..3),
+// summed in the epilogue: tcgen05.mma orders successive products only where
+// accumulator and shape are the same, so windows of different products may not
+// overlap. Wider tiles read X less often but clip
+// T's window, and came out behind. The T blocks (4 KB a chunk) come through a
 // ring of bulk copies from L2, requested by one warp and multiplied by another,
 // whose loop is uniform over the warp.
 #include <cuda_runtime.h>
@@ -64,13 +73,14 @@ constexpr int kPart = kTX / 2;         // output columns per epilogue thread
 // requests the T blocks.
 constexpr int kEpiWarps = 8, kStageWarps = 8, kMmaWarp = 16, kMmaWarps = 2, kLoadWarp = kMmaWarp + kMmaWarps;
 constexpr int kThreads = 32 * (kLoadWarp + 1);
-constexpr int kStages = 6;             // T blocks in flight
+constexpr int kPlanes = 4;             // bytes of a value
 // Tensor-memory columns of one issuing warp's accumulators: X0's levels 0..2
-// from column 0, X1's 1..3 from 96, X2's 2..3 from 192. Sets: kMmaWarps for each
+// from column 0, X1's 1..3 from 96, X2's and X3's 2..3 from 192. Sets: kMmaWarps for each
 // of kBufs tiles (or kernels) in flight.
 constexpr uint32_t kCols = 512, kAccX1 = 3 * kTX, kAccX2 = 6 * kTX, kAccCols = 8 * kTX;
 constexpr uint32_t kBufs = kCols / (kAccCols * kMmaWarps);
-constexpr uint32_t kChunk = 96u * 32u; // bytes of one chunk's T: 96 rows of 32 k
+constexpr uint32_t kChunk = 128u * 32u;  // bytes of one chunk's T: 128 rows (zeros, then three byte planes) of 32 k
+constexpr uint32_t kZeros = kTX * 16u;   // bytes of a half chunk's zero rows
 constexpr int kTurn = kPart + 4;       // pitch (floats) of the rows an epilogue warp turns A and A' in
 constexpr uint32_t kPolls = 1u << 20;  // polls of a barrier before a CTA gives up (about a second)
 
@@ -125,9 +135,10 @@ __device__ __forceinline__ void mma_row(uint32_t tmem, uint32_t a, uint32_t b, u
     for (int c = 0; c <= NQ; ++c) {
         const uint32_t ac = a + uint32_t(c) * (STEP / 16), bc = b + uint32_t(c) * (kChunk / 16);
         const uint32_t add = c > 0 ? 1u : acc;
-        mma_i8(tmem, ac, bc, idesc(96), add, lead);
-        mma_i8(tmem + kAccX1, ac + PLANE / 16, bc, idesc(96), add, lead);
-        mma_i8(tmem + kAccX2, ac + 2 * (PLANE / 16), bc, idesc(64), add, lead);
+        mma_i8(tmem, ac, bc + kZeros / 16, idesc(96), add, lead);
+        mma_i8(tmem + kAccX1, ac + PLANE / 16, bc + kZeros / 16, idesc(96), add, lead);
+        mma_i8(tmem + kAccX2, ac + 2 * (PLANE / 16), bc + kZeros / 16, idesc(64), add, lead);
+        mma_i8(tmem + kAccX2, ac + 3 * (PLANE / 16), bc, idesc(64), 1, lead);
     }
 }
 __device__ __forceinline__ void bar_init(uint64_t* bar, uint32_t count) {
@@ -191,15 +202,16 @@ __device__ __forceinline__ bool out_of_range(const float4& a) {
     return (((__float_as_uint(a.x) | __float_as_uint(a.y)) | (__float_as_uint(a.z) | __float_as_uint(a.w))) &
             0xC0000000u) != 0u;
 }
-// Four values as the bytes of levels 0, 1 and 2, value i in byte i.
-__device__ __forceinline__ void pack_bytes(const float4& a, uint32_t (&w)[3]) {
-    const uint32_t v0 = __float2uint_rn(a.x * 8388608.0f), v1 = __float2uint_rn(a.y * 8388608.0f);
-    const uint32_t v2 = __float2uint_rn(a.z * 8388608.0f), v3 = __float2uint_rn(a.w * 8388608.0f);
+// Four values as the bytes of levels 0 to 3, value i in byte i.
+__device__ __forceinline__ void pack_bytes(const float4& a, uint32_t (&w)[kPlanes]) {
+    const uint32_t v0 = __float2uint_rn(a.x * 2147483648.0f), v1 = __float2uint_rn(a.y * 2147483648.0f);
+    const uint32_t v2 = __float2uint_rn(a.z * 2147483648.0f), v3 = __float2uint_rn(a.w * 2147483648.0f);
     const uint32_t l01 = __byte_perm(v0, v1, 0x5140), l23 = __byte_perm(v2, v3, 0x5140);
     const uint32_t h01 = __byte_perm(v0, v1, 0x7362), h23 = __byte_perm(v2, v3, 0x7362);
-    w[0] = __byte_perm(h01, h23, 0x5410);
-    w[1] = __byte_perm(l01, l23, 0x7632);
-    w[2] = __byte_perm(l01, l23, 0x5410);
+    w[0] = __byte_perm(h01, h23, 0x7632);
+    w[1] = __byte_perm(h01, h23, 0x5410);
+    w[2] = __byte_perm(l01, l23, 0x7632);
+    w[3] = __byte_perm(l01, l23, 0x5410);
 }
 
 // One output of the FP32 form (values the byte form cannot hold): taps in
@@ -218,9 +230,13 @@ __device__ __noinline__ float direct_point(const float* __restrict__ src, const 
     return acc;
 }
 
+// T blocks in flight: what the staged tiles leave room for.
+template <int P>
+constexpr int kStages = P == 16 ? 6 : 5;
+
 // Barriers and flags of a CTA.
 struct TcShared {
-    uint64_t t_full[kStages], t_empty[kStages];  // T blocks
+    uint64_t t_full[6], t_empty[6];              // T blocks
     uint64_t a_full[2], a_empty[2];              // staged halo tiles
     uint64_t d_full[kBufs], d_empty[kBufs];      // accumulators
     uint64_t drain[kMmaWarps];                   // products in flight when a wait ran out
@@ -247,11 +263,11 @@ __global__ void __launch_bounds__(kThreads, 1)
     constexpr uint32_t kStage = kChunk * uint32_t(1 + P / 16);
     const int tid = int(threadIdx.x), warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int W = int(p.width), H = int(p.height);
-    unsigned char* ring = sm + 6u * kPlane;
+    unsigned char* ring = sm + 2u * kPlanes * kPlane;
 
     if (tid == 0) {
         sh.stop = 0;
-        for (int i = 0; i < kStages; ++i) {
+        for (int i = 0; i < kStages<P>; ++i) {
             bar_init(&sh.t_full[i], 1);
             bar_init(&sh.t_empty[i], 1);
         }
@@ -280,7 +296,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     const uint32_t tmem = __shfl_sync(0xffffffffu, sh.tmem, 0);
 
     if (warp >= kEpiWarps && warp < kEpiWarps + kStageWarps) {
-        // ---- Stage the halo tiles as three byte planes, [16-column granule]
+        // ---- Stage the halo tiles as byte planes, [16-column granule]
         // [row][16 bytes]: a warp access covers eight rows of a granule, four
         // lanes a row (64 bytes loaded; the 4-byte stores fill 128 contiguous
         // bytes), five or six accesses in flight.
@@ -294,7 +310,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (ai >= 2 && !bar_wait(&sh.a_empty[buf], ((ai >> 1) - 1u) & 1u, &sh.stop)) break;
             const int ty = tile / tiles_x, x0 = (tile - ty * tiles_x) * kTX, y0 = ty * kRows;
             const bool inside = W % 4 == 0 && x0 >= P && x0 + kTX + P <= W;
-            unsigned char* planes = sm + buf * 3u * kPlane;
+            unsigned char* planes = sm + buf * kPlanes * kPlane;
             bool bad = false;
             if (W % 4 != 0 && x0 >= P && x0 + kTX + P + 3 <= W) {
                 // Rows start anywhere in a 16-byte quad: the quads that hold the
@@ -313,7 +329,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                     for (int f = 0; f < NG; ++f) a[f] = __ldg(quad + 4 * f);
                     // The quad after the last granule's: the group's first lane reads it for the last.
                     a[NG] = (lane & 3) == 0 && shift != 0u ? __ldg(quad + 4 * NG) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    uint32_t w[NG + 1][3];
+                    uint32_t w[NG + 1][kPlanes];
 #pragma unroll
                     for (int f = 0; f <= NG; ++f) {
                         bad = bad || out_of_range(a[f]);
@@ -324,7 +340,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
                     for (int f = 0; f < NG; ++f)
 #pragma unroll
-                        for (int j = 0; j < 3; ++j) {
+                        for (int j = 0; j < kPlanes; ++j) {
                             const uint32_t next =
                                 __shfl_sync(0xffffffffu, (lane & 3) == 0 ? w[f + 1][j] : w[f][j], from);
                             *reinterpret_cast<uint32_t*>(planes + uint32_t(j) * kPlane + (f * RA + row) * 16 + q) =
@@ -353,11 +369,11 @@ __global__ void __launch_bounds__(kThreads, 1)
                 for (int f = 0; f < kFlight; ++f) {
                     const int i = i0 + f * kStageWarps, gran = i / kGroups, row = (i - gran * kGroups) * 8 + rl;
                     bad = bad || out_of_range(a[f]);
-                    uint32_t w[3];
+                    uint32_t w[kPlanes];
                     pack_bytes(a[f], w);
                     unsigned char* o = planes + (gran * RA + row) * 16 + q;
 #pragma unroll
-                    for (int j = 0; j < 3; ++j) *reinterpret_cast<uint32_t*>(o + uint32_t(j) * kPlane) = w[j];
+                    for (int j = 0; j < kPlanes; ++j) *reinterpret_cast<uint32_t*>(o + uint32_t(j) * kPlane) = w[j];
                 }
             }
             }
@@ -374,8 +390,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             uint32_t offset = 0;
 #pragma unroll 1
             for (int r = 0; r < plan.first[nk]; ++r, ++ti) {
-                const uint32_t st = ti % kStages, bytes = kChunk * (1u + (uint32_t(plan.rows[r]) >> 14));
-                if (ti >= kStages && !bar_wait(&sh.t_empty[st], (ti / kStages - 1u) & 1u, &sh.stop)) break;
+                const uint32_t st = ti % kStages<P>, bytes = kChunk * (1u + (uint32_t(plan.rows[r]) >> 14));
+                if (ti >= kStages<P> && !bar_wait(&sh.t_empty[st], (ti / kStages<P> - 1u) & 1u, &sh.stop)) break;
                 if (lane == 0) bulk_load(ring + st * kStage, plan.blocks + offset, bytes, &sh.t_full[st]);
                 offset += bytes;
             }
@@ -384,8 +400,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         // After a wait ran out: the copies in flight get one more bounded wait.
         if (*reinterpret_cast<volatile int*>(&sh.stop)) {
             int never = 0;
-            for (uint32_t i = ti > kStages ? ti - kStages : 0; i < ti; ++i)
-                bar_wait_slow(&sh.t_full[i % kStages], (i / kStages) & 1u, &never);
+            for (uint32_t i = ti > kStages<P> ? ti - kStages<P> : 0; i < ti; ++i)
+                bar_wait_slow(&sh.t_full[i % kStages<P>], (i / kStages<P>) & 1u, &never);
         }
     } else if (warp >= kMmaWarp && warp < kMmaWarp + kMmaWarps) {
         // ---- Products of every kMmaWarps-th T block.
@@ -396,7 +412,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         bool ok = true;
         for (int tile = int(blockIdx.x); tile < tiles && ok; tile += int(gridDim.x), ++ai) {
             const uint32_t buf = ai & 1u;
-            const uint32_t a_base = desc_lo(smem_u32(sm) + buf * 3u * kPlane, RA * 16u) + uint32_t((P / 16) * RA);
+            const uint32_t a_base = desc_lo(smem_u32(sm) + buf * kPlanes * kPlane, RA * 16u) + uint32_t((P / 16) * RA);
             ok = bar_wait(&sh.a_full[buf], (ai >> 1) & 1u, &sh.stop);
 #pragma unroll 1
             for (int k = 0; k < nk && ok; ++k, ++di) {
@@ -426,7 +442,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                         acc = 1;
                         commit(&sh.t_empty[st], lead);
                     }
-                    if (++st == kStages) st = 0, ph ^= 1u;
+                    if (++st == kStages<P>) st = 0, ph ^= 1u;
                 }
                 if (ok) commit(&sh.d_full[db], lead);
             }
@@ -539,7 +555,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
             }
             if (!ok) break;  // its tile is left unwritten
-            float* rows = reinterpret_cast<float*>(ring + kStages * kStage) + warp * (32 * kTurn);
+            float* rows = reinterpret_cast<float*>(ring + kStages<P> * kStage) + warp * (32 * kTurn);
             float4* own = reinterpret_cast<float4*>(rows + lane * kTurn);
             if (!whole) {
 #pragma unroll
@@ -605,7 +621,7 @@ template <int P>
 cudaError_t launch_t(int nk, const float* src, float* dst, const DirectTcPlan& plan, const float* weights,
                      const uint32_t* spans, const DirectGeometry& g, const StepParams& p, int* err, cudaStream_t s) {
     auto fn = direct_tc_kernel<P>;
-    constexpr size_t smem = 6 * size_t(kRows + 2 * P) * (kTX + 2 * P) + size_t(kStages) * kChunk * (1 + P / 16) +
+    constexpr size_t smem = 2 * kPlanes * size_t(kRows + 2 * P) * (kTX + 2 * P) + size_t(kStages<P>) * kChunk * (1 + P / 16) +
                             sizeof(float) * kEpiWarps * 32 * kTurn;
     static fastfft::KernelState state;
     int per = 0;
@@ -620,7 +636,8 @@ cudaError_t launch_t(int nk, const float* src, float* dst, const DirectTcPlan& p
 
 // The T blocks of the kernel tables ((2r + 1)^2 weights each) in the order of
 // the plan's rows: per kernel row with a nonzero weight and per chunk, two
-// halves of k x 96 rows (byte plane j, output n) x 16 values of k.
+// halves of k x 128 rows (32 of zeros, then byte plane j, output n) x 16 values
+// of k.
 bool direct_tc_tables(const std::vector<std::vector<float>>& luts, int r, DirectTcTables& out) {
     out = DirectTcTables();
     if (r < 0 || r > kMaxRadius || luts.empty() || luts.size() > size_t(kMaxKernels)) return false;
@@ -682,7 +699,7 @@ bool direct_tc_tables(const std::vector<std::vector<float>>& luts, int r, Direct
                         const int32_t d[3] = {d0, d1, d2};
                         for (int j = 0; j < 3; ++j)
                             out.blocks[at + size_t(c) * kChunk + size_t(kk / 16) * (kChunk / 2) +
-                                       size_t(j * kTX + n) * 16 + size_t(kk % 16)] = uint8_t(int8_t(d[j]));
+                                       kZeros + size_t(j * kTX + n) * 16 + size_t(kk % 16)] = uint8_t(int8_t(d[j]));
                     }
             out.chunks += (1 + nq) * (same && twin != dyi ? 2 : 1);
             out.plan.rows[rows++] = uint16_t(dyi | ((same ? twin : dyi) << 7) | (nq << 14));
@@ -727,6 +744,14 @@ bool direct_tc_faster(const DirectTcTables& t, uint64_t fp32_taps, int w, int h,
     const double work = px * (double(fp32_taps) * 3.7e-8 + 5e-6);  // of the FP32 form, the SMs full
     const double fp32 = 7.0 + px * (double(fp32_taps) * (px < 1.5e6 ? 4.8e-8 : 3.7e-8) + 5e-6);
     return bytes + share < fp32 + work && bytes < 1.1 * fp32;
+}
+
+// U is off by up to 2^-32 where FP32 values are fainter than 2^-8; FP32 rounds
+// U - mu at 2^-25 |mu| or more there (at mu = 2^-6 twice the former).
+bool direct_tc_holds(int nk, const StepParams& p) {
+    for (int k = 0; k < nk; ++k)
+        if (!(std::fabs(p.mu[k]) >= 0.015625f)) return false;
+    return true;
 }
 
 cudaError_t launch_direct_tc(int nk, const float* src, float* dst, const DirectTcPlan& plan, const float* weights,

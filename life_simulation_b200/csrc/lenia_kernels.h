@@ -88,6 +88,9 @@ bool direct_tc_tables(const std::vector<std::vector<float>>& luts, int r, Direct
 // Whether the tensor-core step is the one to run on a w x h field, against
 // launch_direct_step, which executes fp32_taps multiply-adds a pixel.
 bool direct_tc_faster(const DirectTcTables& t, uint64_t fp32_taps, int w, int h, int sms);
+// Whether the byte form's sums are as close as the FP32 form's for a substep's
+// growth centres (not for centres near zero, where faint potentials count).
+bool direct_tc_holds(int nk, const StepParams& p);
 // weights / spans / g: the FP32 tables (tiles whose values have no byte form
 // use them). err counts CTAs whose wait ran out.
 cudaError_t launch_direct_tc(int nk, const float* src, float* dst, const DirectTcPlan& plan, const float* weights,

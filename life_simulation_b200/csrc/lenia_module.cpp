@@ -1433,7 +1433,7 @@ int LeniaModule::stepImpl(const lenia_frame_params& fp, uint32_t substeps, cudaS
             spectrum_valid_ = true;
         } else {
             e = launch(LENIA_PHASE_DIRECT, s, [&] {
-                if (direct_tc_on_)
+                if (direct_tc_on_ && direct_tc_holds(direct_nk_, p))
                     return launch_direct_tc(direct_nk_, src, dst, direct_tc_, d_weights_, d_spans_, dgeo_, p, d_tma_err_,
                                             s);
                 return launch_direct_step(direct_tile_, direct_nk_, src, dst, d_weights_, d_spans_, dgeo_, p, s,
