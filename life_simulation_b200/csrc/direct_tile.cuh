@@ -140,11 +140,8 @@ __device__ __forceinline__ void stage_wrapped(float* tile, int TR, int TP, const
 // splits the kernel rows over S thread groups (group s takes rows dy = s,
 // s + S, ...) for fields too small to fill the GPU one thread per 8 outputs:
 // the groups' partial sums meet in shared memory and are added in group
-// order before the epilogue. IEEE (one kernel): the growth map with a division
-// by sigma and the full-range exponential, as a batch's worlds take it: a sweep
-// runs thousands of substeps, over which its fields amplify a last-place
-// difference, and the map is a small part of a batch tile.
-template <int TW, int TH, int NK, int S = 1, int OX = PX, int OY = 1, bool IEEE = false>
+// order before the epilogue. BATCH: EulerStep::rounded.
+template <int TW, int TH, int NK, int S = 1, int OX = PX, int OY = 1, bool BATCH = false>
 __device__ __forceinline__ void direct_tile(const float* __restrict__ src, float* __restrict__ dst,
                                             const float* __restrict__ weights,  // [NK][2R+1][WP], zero padded
                                             const uint32_t* __restrict__ spans, // [NK][2R+1]
@@ -322,39 +319,15 @@ __device__ __forceinline__ void direct_tile(const float* __restrict__ src, float
         if (gy >= H) return;
         const float* arow = tile + (ty + o + g.r) * TP + ox + g.xp;
         float v[OX];
-        if constexpr (IEEE) {
-            static_assert(NK == 1, "one kernel per world");
+        const uint32_t jrow = p.mu_jitter > 0.0f ? rand_row(uint32_t(gy), ex.jitter_base) : 0u;
 #pragma unroll
-            for (int j = 0; j < OX; ++j) {
-                const float mu = p.mu_jitter > 0.0f
-                                     ? p.mu[0] + mu_jitter_shift(p, uint32_t(x0 + ox + j), rand_row(uint32_t(gy), ex.jitter_base))
-                                     : p.mu[0];
-                const float t = (acc[o][0][j] - mu) / p.sigma[0];
-                const float b = expf(-0.5f * t * t), h = p.weight[0], A = arow[j];
-                if (euler.asym)
-                    v[j] = A + p.dt * ((euler.weighted ? h * b / p.sum_weights : A) - A);
-                else
-                    v[j] = A + p.dt * (h * (2.0f * b - 1.0f));
-            }
-        } else {
-        float2 sum[OX / 2];  // growth sums of pixel pairs
+        for (int j = 0; j < OX; ++j) {
+            const float shift = p.mu_jitter > 0.0f ? mu_jitter_shift(p, uint32_t(x0 + ox + j), jrow) : 0.0f;
+            float sum = 0.0f;
 #pragma unroll
-        for (int k = 0; k < NK; ++k) {
-            const GrowthPair gp(p.mu[k], 1.0f / p.sigma[k], p.weight[k], euler.asym);
-#pragma unroll
-            for (int j = 0; j < OX / 2; ++j) {
-                const float2 u = make_float2(acc[o][k][2 * j], acc[o][k][2 * j + 1]);
-                const float2 c = gp.term_near(
-                    u, p.mu_jitter > 0.0f ? mu_jitter_pair(p, ex, uint32_t(x0 + ox + 2 * j), uint32_t(gy))
-                                          : make_float2(0.0f, 0.0f));
-                sum[j] = k == 0 ? c : __fadd2_rn(sum[j], c);
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < OX / 2; ++j) {
-            v[2 * j] = euler(arow[2 * j], sum[j].x);
-            v[2 * j + 1] = euler(arow[2 * j + 1], sum[j].y);
-        }
+            for (int k = 0; k < NK; ++k)
+                sum = growth_add(sum, p.weight[k], bell(acc[o][k][j], p.mu[k] + shift, p.sigma[k]), euler.asym);
+            v[j] = BATCH ? euler.rounded(arow[j], sum) : euler(arow[j], sum);
         }
         noise_inject_clip(p, ex, v, uint32_t(x0 + ox), uint32_t(gy));
 #pragma unroll

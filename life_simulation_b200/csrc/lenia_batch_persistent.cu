@@ -438,8 +438,8 @@ __global__ void __launch_bounds__(kPT, 2)
             }
         } else {
             const int g = s_it.group;
-            direct_tile<64, 32, 1, 1, 8, 1, true>(s_dw.src, s_dw.dst, s_dw.weights, s_dw.spans, s_dw.g, s_dw.p,
-                                            (g & 0xFFFF) * 64, (g >> 16) * 32, nullptr, nullptr);
+            direct_tile<64, 32, 1, 1, PX, 1, true>(s_dw.src, s_dw.dst, s_dw.weights, s_dw.spans, s_dw.g, s_dw.p,
+                                                   (g & 0xFFFF) * 64, (g >> 16) * 32, nullptr, nullptr);
             tab_kind = -1;  // the tile overwrote the tables
         }
         cur = s_next;

@@ -65,13 +65,17 @@ __device__ __forceinline__ float mu_jitter_shift(const StepParams& p, uint32_t g
     return (rand01_row(gx, row) - 0.5f) * p.mu_jitter * 0.05f;
 }
 
-// bell(u; mu, sigma) = exp(-0.5 t^2), t = (u - mu) / sigma (Lenia.metal:156-159)
-// with a precomputed 1/sigma and one hardware base-2 exponential: 2^(-0.5
-// log2(e) t^2). ex2.approx.ftz has a relative error below 2^-22 (dt times that
-// reaches A, under A's own rounding), and it replaces an IEEE division and the
-// full-range expf sequence: on the direct path these were about 60 of the
-// epilogue's 127 instructions a pixel.
-//
+// bell(u; mu, sigma) = exp(-0.5 t^2), t = (u - mu) / sigma (Lenia.metal:156-159).
+__device__ __forceinline__ float bell(float u, float mu, float sigma) {
+    const float t = (u - mu) / sigma;
+    return expf(-0.5f * t * t);
+}
+// A pixel's growth sum with one more kernel's term, in the reference's order
+// (Lenia.metal:188-195): sum_k h_k bell_k (asymptotic) or sum_k h_k (2 bell_k - 1).
+__device__ __forceinline__ float growth_add(float sum, float h, float b, bool asym) {
+    return fmaf(h, asym ? b : 2.0f * b - 1.0f, sum);
+}
+
 // 2^x by the SFU's approximate base-2 exponential (relative error < 2^-22,
 // subnormal results flushed to zero).
 __device__ __forceinline__ float ex2_fast(float x) {
@@ -80,7 +84,10 @@ __device__ __forceinline__ float ex2_fast(float x) {
     return r;
 }
 
-// One kernel's growth terms at a pixel pair:
+// One kernel's growth terms at a pixel pair of the spectral row passes, where
+// the map is a large share: a precomputed 1/sigma and one hardware base-2
+// exponential (relative error below 2^-22) for the division and the full-range
+// expf of `bell`, under the transforms' own rounding.
 // bell(u) = exp(-(u - mu)^2 / (2 sigma^2)) = 2^-((u*sc - mu*sc)^2) with
 // sc = sqrt(log2(e) / 2) / sigma, and the term h * (2 bell - 1) (growth mode
 // 0) or h * bell (mode 1) as g1 * bell + g0 -- in packed FP32x2 pairs (one
@@ -102,12 +109,6 @@ struct GrowthPair {
     // The same with the pair's mu shifts.
     __device__ __forceinline__ float2 term(float2 u, float2 shift) const {
         return bells(make_float2((u.x - (mu + shift.x)) * sc, (u.y - (mu + shift.y)) * sc));
-    }
-    // The same, its difference u - mu taken first (exact near mu): the direct
-    // paths' potentials carry less rounding than the transforms', and u * sc -
-    // mu * sc would add that of mu * sc.
-    __device__ __forceinline__ float2 term_near(float2 u, float2 shift) const {
-        return bells(__fmul2_rn(__fadd2_rn(u, make_float2(-(mu + shift.x), -(mu + shift.y))), SC));
     }
     // d: (u - mu) * sc for both pixels.
     __device__ __forceinline__ float2 bells(float2 d) const {
@@ -131,9 +132,12 @@ struct EulerStep {
     bool asym, weighted;
     __device__ __forceinline__ explicit EulerStep(const StepParams& p)
         : dt(p.dt), inv_sum(1.0f / p.sum_weights), asym(p.growth_mode == 1u), weighted(p.sum_weights > 1e-6f) {}
-    __device__ __forceinline__ float operator()(float A, float s) const {
-        return asym ? A + dt * ((weighted ? s * inv_sum : A) - A) : A + dt * s;
-    }
+    // dA / dt.
+    __device__ __forceinline__ float rate(float A, float s) const { return asym ? (weighted ? s * inv_sum : A) - A : s; }
+    __device__ __forceinline__ float operator()(float A, float s) const { return fmaf(dt, rate(A, s), A); }
+    // With its product rounded before the sum: how a batch's direct worlds have always
+    // stepped, and over a sweep's thousands of substeps a field amplifies a last place.
+    __device__ __forceinline__ float rounded(float A, float s) const { return __fadd_rn(A, __fmul_rn(dt, rate(A, s))); }
 };
 
 // Noise stir, blob injection and clip (Lenia.metal:210-231) of the N pixels

@@ -486,7 +486,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 for (int c = 0; c < kPart; ++c)
                     av[c] = x < W ? __ldg(src + size_t(min(gq + 2 * c + (lane >> 4), H - 1)) * W + x) : 0.0f;
             }
-            float2 sum[kPart / 2];  // growth sums of pixel pairs
+            float sum[kPart] = {};  // growth sums
 #pragma unroll 1
             for (int k = 0; k < nk; ++k, ++di) {
                 const uint32_t db = di % kBufs;
@@ -495,7 +495,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const bool bytes = *reinterpret_cast<volatile int*>(&sh.bad[ai & 3u]) != int(ai) + 1;
                 const float scale = pick(plan.scale, k);
                 const float s0 = scale * 512.0f, s1 = scale * 2.0f;
-                const GrowthPair gp(pick(p.mu, k), 1.0f / pick(p.sigma, k), pick(p.weight, k), euler.asym);
+                const float mu = pick(p.mu, k), sigma = pick(p.sigma, k), weight = pick(p.weight, k);
                 // T blocks of kernel k: the issuing warps that had one.
                 const int blocks = plan.first[k + 1] - plan.first[k];
                 float u[kPart];
@@ -547,11 +547,11 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
 #pragma unroll
                 for (int j = 0; j < kPart / 2; ++j) {
-                    const float2 uu = make_float2(u[2 * j], u[2 * j + 1]);
-                    const float2 t =
-                        gp.term_near(uu, jitter ? mu_jitter_pair(p, sh.ex, uint32_t(gx0 + 2 * j), uint32_t(gy))
-                                                : make_float2(0.0f, 0.0f));
-                    sum[j] = k == 0 ? t : __fadd2_rn(sum[j], t);
+                    const float2 shift = jitter ? mu_jitter_pair(p, sh.ex, uint32_t(gx0 + 2 * j), uint32_t(gy))
+                                                : make_float2(0.0f, 0.0f);
+                    sum[2 * j] = growth_add(sum[2 * j], weight, bell(u[2 * j], mu + shift.x, sigma), euler.asym);
+                    sum[2 * j + 1] =
+                        growth_add(sum[2 * j + 1], weight, bell(u[2 * j + 1], mu + shift.y, sigma), euler.asym);
                 }
             }
             if (!ok) break;  // its tile is left unwritten
@@ -573,10 +573,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (int c = 0; c < kPart; c += 8) {
                 float v[8];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    v[2 * j] = euler(av[c + 2 * j], sum[c / 2 + j].x);
-                    v[2 * j + 1] = euler(av[c + 2 * j + 1], sum[c / 2 + j].y);
-                }
+                for (int j = 0; j < 8; ++j) v[j] = euler(av[c + j], sum[c + j]);
                 noise_inject_clip(p, sh.ex, v, uint32_t(gx0 + c), uint32_t(gy));
                 const float4 lo = make_float4(v[0], v[1], v[2], v[3]), hi = make_float4(v[4], v[5], v[6], v[7]);
                 if (!whole) {
