@@ -125,15 +125,14 @@ __device__ __forceinline__ float bell_fast(float u, float mu, float inv_sigma) {
 
 // Euler step (Lenia.metal:197-209, identical to leniaStep's for one kernel of
 // weight 1); s: the mode's growth sum, sum_k h_k * bell_k (asymptotic) or
-// sum_k h_k * (2 bell_k - 1), in kernel order (Lenia.metal:188-195). The
-// division by sum_k h_k is a product with its reciprocal, taken once.
+// sum_k h_k * (2 bell_k - 1), in kernel order (Lenia.metal:188-195).
 struct EulerStep {
-    float dt, inv_sum;
+    float dt, sum_weights;
     bool asym, weighted;
     __device__ __forceinline__ explicit EulerStep(const StepParams& p)
-        : dt(p.dt), inv_sum(1.0f / p.sum_weights), asym(p.growth_mode == 1u), weighted(p.sum_weights > 1e-6f) {}
+        : dt(p.dt), sum_weights(p.sum_weights), asym(p.growth_mode == 1u), weighted(p.sum_weights > 1e-6f) {}
     // dA / dt.
-    __device__ __forceinline__ float rate(float A, float s) const { return asym ? (weighted ? s * inv_sum : A) - A : s; }
+    __device__ __forceinline__ float rate(float A, float s) const { return asym ? (weighted ? s / sum_weights : A) - A : s; }
     __device__ __forceinline__ float operator()(float A, float s) const { return fmaf(dt, rate(A, s), A); }
     // With its product rounded before the sum: how a batch's direct worlds have always
     // stepped, and over a sweep's thousands of substeps a field amplifies a last place.

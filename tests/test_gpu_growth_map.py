@@ -37,3 +37,21 @@ def test_far_tail_of_the_bell(monkeypatch, engine, conv):
     # bell at 2^-149.
     assert 1e-3 < expected < 0.5
     assert abs(got - expected) <= expected * (t / float(sigma) * 0.31 * 80 * 2.0**-24 + 1e-5) + float(dt) * 2.0**-149
+
+
+@pytest.mark.parametrize("weight", [0.42, 0.77, 41.0])
+@pytest.mark.parametrize("w,h,conv,engine", [(96, 64, "directMulti", "ffma"), (131, 150, "directMulti", "tensor"),
+                                             (256, 128, "fft", ""), (512, 72, "fft", ""), (90, 75, "fft", ""),
+                                             (60, 60, "fft", "")])
+def test_the_weights_sum_divides(monkeypatch, w, h, conv, engine, weight):
+    """A kernel so wide that its bell is one everywhere: the target is h / h, which
+    a division gives as exactly one and a product with 1 / h does not."""
+    assert np.float32(weight) * (np.float32(1.0) / np.float32(weight)) != np.float32(1.0)
+    p = {"convMode": conv, "fftAnySize": True, "radius": 9, "growthMode": 1, "dt": 1.0,
+         "kernels": [{"radiusScale": 1.0, "mu": 0.2, "sigma": 1e6, "weight": weight, "betas": [1.0]}]}
+    m = module(monkeypatch, engine, p, w, h)
+    assert not m.warning
+    m.upload(np.zeros((h, w), np.float32))
+    m.encode(0, 1)
+    np.testing.assert_array_equal(m.field(), np.float32(1.0))
+    m.close()
