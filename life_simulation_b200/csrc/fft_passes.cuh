@@ -2,7 +2,7 @@
 // row pass kernels for transform lengths with a compile-time FFT plan, and
 // their launches: instantiated by lenia_fft_fast.cu for the catalogue's sizes
 // (several launch shapes each) and by lenia_fft_wide*.cu for every other
-// length with factors 2, 3 and 5 in their range (one shape each).
+// length with factors 2, 3 and 5 in their range (two shapes each).
 //
 // Spectral layout of this path ("blocked"): spectra S and U_k are stored in
 // blocks of 8 columns, element (kx, ky) at ((kx/8)*H + ky)*8 + kx%8, so a row
@@ -269,7 +269,10 @@ static __device__ __noinline__ void palette_pair(const ColorMapParams& cm, float
 // (one staging buffer, which doubles as the second work buffer) each item is
 // staged and waited for in turn: less shared memory per CTA, which wins
 // where shared memory limits the resident CTAs (long rows).
-template <class PI, int RB, bool PIPE, bool CM, int SPLIT>
+//
+// NEAR: the growth terms by GrowthPair::term_near (the wide lengths, whose
+// sizes the runtime plan served with the full-range map).
+template <class PI, int RB, bool PIPE, bool CM, int SPLIT, bool NEAR>
 __global__ void __launch_bounds__(RowK<PI, RB, SPLIT>::T,
                                   (512 / RowK<PI, RB, SPLIT>::T > 1 ? 512 / RowK<PI, RB, SPLIT>::T : 1))
     row_fast_kernel(SpectralWorld w0, const SpectralWorld* __restrict__ worlds,
@@ -383,8 +386,12 @@ __global__ void __launch_bounds__(RowK<PI, RB, SPLIT>::T,
                 }
 #pragma unroll
                 for (int t = 0; t < RC; ++t) {
-                    const float2 c = jitter ? gp.term(z[t], mu_jitter_pair(p, ex, uint32_t(2 * (jj[it] + t * NRC)), gy))
-                                            : gp.term(z[t]);
+                    const auto shift = [&] { return mu_jitter_pair(p, ex, uint32_t(2 * (jj[it] + t * NRC)), gy); };
+                    float2 c;
+                    if constexpr (NEAR)
+                        c = gp.term_near(z[t], jitter ? shift() : make_float2(0.0f, 0.0f));
+                    else
+                        c = jitter ? gp.term(z[t], shift()) : gp.term(z[t]);
                     acc[it][t] = kk == 0 ? c : __fadd2_rn(acc[it][t], c);
                 }
             }
@@ -475,11 +482,11 @@ cudaError_t launch_col_t(const SpectralWorld& w0, const SpectralWorld* worlds, i
     return launch_chained(fn, world_grid(per, (M + B - 1) / B, n), K::T, smem, s, w0, worlds, t.col_twf, t.col_twi);
 }
 
-template <class PI, int RB, bool PIPE, bool CM, int S = 1>
+template <class PI, int RB, bool PIPE, bool CM, int S = 1, bool NEAR = false>
 cudaError_t launch_row_t(const SpectralWorld& w0, const SpectralWorld* worlds, int n, int H,
                          const float2* tw_r2c, const FastTables& t, cudaStream_t s) {
     using K = RowK<PI, RB, S>;
-    auto fn = row_fast_kernel<PI, RB, PIPE, CM, S>;
+    auto fn = row_fast_kernel<PI, RB, PIPE, CM, S, NEAR>;
     const size_t smem = K::smem(PIPE ? 3 : 2);
     if (smem > 227 * 1024) return cudaErrorInvalidConfiguration;
     static KernelState state;

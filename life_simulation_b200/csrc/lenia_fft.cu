@@ -188,12 +188,14 @@ __global__ void row_c2r_growth_kernel(FftGeometry g, const float2* __restrict__ 
             }
             __syncthreads();
             const float2* z = fft::run<true>(bb, ba, g.row, rows, tw);
-            const GrowthPair gp(p.mu[kk], 1.0f / p.sigma[kk], p.weight[kk], asym);
+            const float mu = p.mu[kk], sigma = p.sigma[kk], h = p.weight[kk];
             for (int q = threadIdx.x; q < M * rows; q += blockDim.x) {
                 const int r = q / M, n = q - r * M;
-                const float2 c = jitter ? gp.term(z[q], mu_jitter_pair(p, ex, uint32_t(2 * n), uint32_t(y0 + r)))
-                                        : gp.term(z[q]);
+                const float2 shift = jitter ? mu_jitter_pair(p, ex, uint32_t(2 * n), uint32_t(y0 + r))
+                                            : make_float2(0.0f, 0.0f);
                 float2* ar = reinterpret_cast<float2*>(acc) + q;
+                const float2 c = make_float2(growth_add(0.0f, h, bell(z[q].x, mu + shift.x, sigma), asym),
+                                             growth_add(0.0f, h, bell(z[q].y, mu + shift.y, sigma), asym));
                 *ar = kk == 0 ? c : __fadd2_rn(*ar, c);
             }
             __syncthreads();

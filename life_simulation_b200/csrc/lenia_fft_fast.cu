@@ -1,7 +1,7 @@
 // life_simulation_b200/csrc/lenia_fft_fast.cu -- the spectral path's column
 // and row passes for field sizes with a compile-time FFT plan (the sizes of
-// the benchmark configs and common sim resolutions; other sizes use the
-// runtime-plan kernels of lenia_fft.cu).
+// the benchmark configs and common sim resolutions; the other lengths with
+// factors 2, 3 and 5 are lenia_fft_wide*.cu's, the rest lenia_fft.cu's).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -240,8 +240,7 @@ cudaError_t launch_row_wide(const FftGeometry& g, const FastTables& t, int shape
                             const ColorMapParams* cm) {
     const SpectralWorld w = row_world(g, U, A, A_out, S_next, p, nk, rgba16f, cm);
     FastPlan catalogue;
-    if (fast_row_plan(g.M, catalogue))
-        return row_dispatch(g.H, g.M, (shape == 0 ? 4 : 2) | kRowPipelined, w, nullptr, 1, g.tw_r2c, t, s);
+    if (fast_row_plan(g.M, catalogue)) return wide_row_mixed(g.M, g.H, shape, w, g.tw_r2c, t, s);
     cudaError_t e = cudaErrorNotSupported;
 #define F(p_) \
     if (e == cudaErrorNotSupported) e = wide_row_##p_(g.M, g.H, shape, w, g.tw_r2c, t, s);

@@ -147,5 +147,9 @@ constexpr int wide_rows() {
 #define LENIA_WIDE_EACH(F) F(0) F(1) F(2) F(3) F(4) F(5) F(6) F(7)
 LENIA_WIDE_EACH(LENIA_WIDE_DECLARE)
 #undef LENIA_WIDE_DECLARE
+// The row passes of the catalogue's half rows under a wide column length
+// (lenia_fft_wide_mixed.cu): the catalogue's plans, the wide lengths' growth map.
+cudaError_t wide_row_mixed(int M, int H, int shape, const SpectralWorld& w, const float2* tw_r2c, const FastTables& t,
+                           cudaStream_t s);
 
 }  // namespace lenia

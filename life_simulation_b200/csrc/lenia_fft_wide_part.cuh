@@ -53,8 +53,8 @@ template <class PI, bool CM>
 cudaError_t wide_row_shape(int H, int shape, const SpectralWorld& w, const float2* tw_r2c, const FastTables& t,
                            cudaStream_t s) {
     constexpr int RB = wide_rows<PI>();
-    if (shape == 0) return launch_row_t<PI, RB, true, CM>(w, nullptr, 1, H, tw_r2c, t, s);
-    if constexpr (RB > 1) return launch_row_t<PI, RB / 2, true, CM>(w, nullptr, 1, H, tw_r2c, t, s);
+    if (shape == 0) return launch_row_t<PI, RB, true, CM, 1, true>(w, nullptr, 1, H, tw_r2c, t, s);
+    if constexpr (RB > 1) return launch_row_t<PI, RB / 2, true, CM, 1, true>(w, nullptr, 1, H, tw_r2c, t, s);
     return cudaErrorNotSupported;
 }
 
