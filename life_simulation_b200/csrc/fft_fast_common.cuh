@@ -343,14 +343,13 @@ inline int sms() {
     return n;
 }
 
-// Opts a kernel into `smem` bytes of dynamic shared memory and the largest
-// shared-memory carveout, and gives its resident CTAs per SM at `threads`
-// threads. A kernel's answer depends on the device alone (each instantiation
-// launches with one shape, or has a state for each and a common `limit`), so
-// `state` keeps it per device: asked on every launch, the three driver calls cost host time that a
-// small field's frame waits for (with the parameter keys spelled out once, an
-// encode of one substep of 64 x 64 went from 8.5 to 7.0 us on the spectral
-// path and from 5.6 to 4.5 us on the direct one, both then bound by the GPU).
+// Opts a kernel into `smem` (at least `limit`) bytes of dynamic shared memory
+// and the largest shared-memory carveout, and gives its resident CTAs per SM at
+// `threads` threads. The opt-in belongs to the CUDA context, so it is made for
+// every launch (two calls of 54 ns): a context that follows a device reset, or
+// a second one on the device, has none of an earlier one's. The resident CTAs
+// depend on the device alone (each instantiation launches with one shape, or has a
+// state for each and a common `limit`), so `state` keeps them per device.
 struct KernelState {
     static constexpr int kDevices = 32;
     std::atomic<int> per_sm[kDevices] = {};  // resident CTAs + 1; 0: not asked yet
@@ -360,11 +359,11 @@ cudaError_t prepare(KernelState& state, F fn, int threads, size_t smem, int& per
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    const bool kept = dev >= 0 && dev < KernelState::kDevices;
-    if (kept && (per_sm = state.per_sm[dev].load(std::memory_order_acquire) - 1) >= 0) return cudaSuccess;
     e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(std::max(smem, limit)));
     if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     if (e != cudaSuccess) return e;
+    const bool kept = dev >= 0 && dev < KernelState::kDevices;
+    if (kept && (per_sm = state.per_sm[dev].load(std::memory_order_acquire) - 1) >= 0) return cudaSuccess;
     per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem);
     if (kept) state.per_sm[dev].store(per_sm + 1, std::memory_order_release);

@@ -24,10 +24,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cstdint>
 #include <cstring>
-#include <mutex>
 
 #include "direct_tile.cuh"
 #include "fft_fast_common.cuh"
@@ -38,7 +36,8 @@ namespace lenia {
 
 namespace {
 
-constexpr int kOptedDevices = 32;
+// A CTA's shared memory (227 KB) less what these kernels declare statically.
+constexpr int kDirectSmemLimit = 226 * 1024;
 
 template <int TW, int TH, int NK, int S, int OX, int OY>
 __global__ void __launch_bounds__(DirectTile<TW, TH, OX, OY>::kThreads * S)
@@ -72,23 +71,10 @@ cudaError_t launch_t(const float* src, float* dst, const float* weights, const u
                         sizeof(uint32_t) * NK * g.ksize +
                         sizeof(float) * size_t(S - 1) * NK * DirectTile<TW, TH, OX, OY>::kThreads * OX;
     auto fn = direct_step_kernel<TW, TH, NK, S, OX, OY>;
-    // The shared memory this instantiation may use, per device: raised when a
-    // larger radius first needs it (see KernelState in fft_fast_common.cuh).
-    static std::atomic<size_t> opted[kOptedDevices];
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    // The opt-in of every launch is the same, whatever its radius: two threads
+    // must not lower each other's.
+    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kDirectSmemLimit);
     if (e != cudaSuccess) return e;
-    const bool kept = dev >= 0 && dev < kOptedDevices;
-    if (!kept || opted[dev].load(std::memory_order_acquire) < smem) {
-        // Raised under a lock: two threads must not lower each other's limit.
-        static std::mutex raise;
-        const std::lock_guard<std::mutex> hold(raise);
-        if (!kept || opted[dev].load(std::memory_order_acquire) < smem) {
-            e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-            if (e != cudaSuccess) return e;
-            if (kept) opted[dev].store(smem, std::memory_order_release);
-        }
-    }
     CUtensorMap map;
     std::memset(&map, 0, sizeof map);
     const bool on = tma && tma->on && (buffer == 0 || buffer == 1);
