@@ -525,10 +525,26 @@ size_t persist_smem_bytes(const std::vector<int>& col_h, const std::vector<int>&
     return s;
 }
 
+// The opt-in is the largest any batch needs, not this batch's: a batch of
+// smaller worlds must not lower another's between its captures.
+cudaError_t persist_opt_in() {
+    static const int limit = [] {
+        std::vector<int> col_h, row_m;
+#define X(n, ...) col_h.push_back(n);
+        LENIA_PERSIST_COLS(X)
+#undef X
+#define X(n, ...) row_m.push_back(n);
+        LENIA_PERSIST_ROWS(X)
+#undef X
+        return int(persist_smem_bytes(col_h, row_m, kMaxRadius));
+    }();
+    cudaError_t e = cudaFuncSetAttribute(persist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(persist_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    return e;
+}
+
 int persist_grid(size_t smem) {
-    if (cudaFuncSetAttribute(persist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
-        return 0;
-    cudaFuncSetAttribute(persist_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    if (persist_opt_in() != cudaSuccess) return 0;
     int per = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, persist_kernel, kPT, smem) != cudaSuccess) return 0;
     return per * fastfft::sms();
@@ -538,6 +554,8 @@ cudaError_t launch_persistent(const PersistItem* items, int nitems, uint32_t* ct
                               StepParams* const* loc, const uint32_t* base_seed, uint32_t* frame, bool advance,
                               int* err, size_t smem, int grid, cudaStream_t s) {
     if (grid <= 0) return cudaErrorInvalidConfiguration;
+    const cudaError_t e = persist_opt_in();
+    if (e != cudaSuccess) return e;
     persist_kernel<<<grid, kPT, smem, s>>>(items, nitems, ctl, nworlds, par, loc, base_seed, frame,
                                            advance ? 1 : 0, err);
     return cudaGetLastError();
