@@ -298,11 +298,14 @@ int lenia_step_render(lenia_ctx* ctx, const lenia_frame_params* fp, uint32_t sub
  * over every direct world plus one column and one row launch per field size
  * with spectral worlds; creation times both and keeps the faster
  * (lenia_batch_launch_form). lenia_batch_step replays k substeps as one
- * captured CUDA graph. The path of
- * each world is chosen at creation: LENIA_BATCH_AUTO gives each world the
- * path whose launches cost it less, by a rule on the batch's sizes and taps
- * (the same for every batch of the same worlds). Each world evolves exactly
- * as it would alone. */
+ * captured CUDA graph. The path of each world is chosen at creation by a rule
+ * on the batch's sizes and taps (LENIA_BATCH_AUTO; the same for every batch of
+ * the same worlds): the path whose launches, each on its own, cost the world
+ * less. The two paths round differently, so for mixed batches of radii above 9 the
+ * rule keeps its line although launches of several sizes overlap: LENIA_BATCH_FFT
+ * is the faster choice for up to a few dozen such worlds. Worlds never interact:
+ * each evolves as it would in a batch of its own on that path.
+ */
 typedef struct lenia_world {
     uint32_t width, height;
     uint32_t radius;          /* kernel radius (px) */

@@ -661,23 +661,37 @@ int lenia_batch_create(const lenia_world* worlds, uint32_t n, uint32_t policy, l
         // Policy AUTO: the path whose launches, each on its own, cost a world
         // less -- the spectral step of its size class, shared by the class's
         // worlds, against its share by pixel-taps of the direct launch over
-        // every world that has both paths. The constants are fitted to what
-        // timing those launches at creation picked (3456 worlds of mixed radii
-        // in batches of 1 to 60: 97 % the same, and 95 % of 1320 batches of one
-        // size and radius; timing disagreed with itself on 1 % between two
-        // processes): 4.74 us a class's two spectral launches, 31.3 fs a
-        // pixel-tap of a full direct launch, and a direct launch no shorter than
-        // 0.52 us and 0.96 us per pixel of its largest radius (a tile's halo and
-        // its threads' chain of taps).
-        // A rule instead of the timing gives a batch the same paths, and so the
-        // same bits, every time. It deliberately keeps the line where the timing
-        // had it, since such fields amplify the two paths' rounding (2e-4 after
-        // 60 substeps on 1 world in 500); for small batches of mixed sizes the
-        // chains run side by side and LENIA_BATCH_FFT is the faster policy
-        // (4 worlds x 60 substeps 1.1 against 1.6 to 1.8 ms, 8 worlds 1.2 against
-        // 1.7 to 2.4; from 48 worlds on they are level).
+        // every world that has both paths. A rule, not a timing at creation, so
+        // that a batch of the same worlds has the same paths, and so the same
+        // bits, every time.
+        //
+        // Radii up to 9: the two launches as measured, uniform batches of 1 to 60
+        // worlds, 128 x 64 to 4096 x 4096, us a substep. Both cost the same per
+        // pixel (7.2 ps) but for the taps, so what decides is the direct launch's
+        // fixed part (4.0 + 0.47 R, a tile's halo and its threads' chain of taps)
+        // and 0.060 ps a pixel-tap against the spectral class's fixed 10.9 us.
+        // The path picked is within 11 % of the better one at each of 372 points,
+        // 0.2 % on average. Direct / spectral:
+        //                  1 world                  8 worlds                 16 worlds
+        //            R 4        6        9          4        6        9         4
+        //   128^2  6.9/10.8 7.8/10.6 10.8/10.7  7.0/11.6 8.3/11.6 11.8/11.6  8.2/12.1
+        //   256^2  6.9/12.4 7.9/13.3 10.7/12.6 11.5/14.2 14.3/13.9 20.9/13.9 15.5/16.7
+        //   512^2  8.1/12.8 10.2/13.2 14.9/12.9 26.9/27.1 35.6/26.8 55.9/25.0 48.9/42.7
+        //   1080p 27.1/27.5 35.8/26.7 55.8/26.7
+        //
+        // Larger radii: constants fitted to what timing those launches at creation
+        // used to pick, on batches of mixed radii and the sizes 128 x 128, 256 x
+        // 256, 384 x 216 and 512 x 512 (3456 worlds: 97 % the same; the timing
+        // disagreed with itself on 1 % between two processes): 4.74 us a class's two
+        // launches, 31.3 fs a pixel-tap, a direct launch no shorter than 0.52 us and
+        // 0.96 us per pixel of its largest radius. That line stays where it is
+        // although the chains now run side by side, since fields amplify the two
+        // paths' rounding (2e-4 after 60 substeps on 1 world in 500): small batches
+        // of mixed sizes are faster under LENIA_BATCH_FFT (4 worlds x 60 substeps
+        // 1.1 against 1.6 to 1.8 ms, 8 worlds 1.2 against 1.7 to 2.4; level from 48
+        // worlds on). At the other sizes above, uniform batches of R = 13 to 32 go
+        // spectral, which is 1.15 to 23 times the faster path there.
         if (policy == LENIA_BATCH_AUTO) {
-            constexpr double kClass = 4.74e-6, kTap = 31.3e-15, kDirect = 0.52e-6, kRadius = 0.961e-6;
             const auto taps = [&](uint32_t i) { return double(worlds[i].width) * worlds[i].height * nnz[i]; };
             double total = 0.0;
             uint32_t largest = 0;
@@ -686,11 +700,19 @@ int lenia_batch_create(const lenia_world* worlds, uint32_t n, uint32_t policy, l
                     total += taps(i);
                     largest = std::max(largest, worlds[i].radius);
                 }
-            const double per_tap = total > 0.0 ? std::max(kTap, (kDirect + kRadius * largest) / total) : kTap;
+            const auto direct_is_cheaper = [&](double world_taps, double members) {
+                if (largest <= 9) {
+                    const double share = total > 0.0 ? world_taps / total : 1.0;
+                    return share * (4.0e-6 + 0.47e-6 * largest) + 0.060e-12 * world_taps <= 10.9e-6 / members;
+                }
+                const double per_tap = std::max(31.3e-15, (0.52e-6 + 0.961e-6 * largest) / total);
+                return world_taps * per_tap <= 4.74e-6 / members;
+            };
             for (uint32_t i = 0; i < n; ++i)
                 if (can_direct[i] && can_fft[i])
-                    b.path[i] = taps(i) * per_tap <= kClass / double(class_members[size_t(cls[i])].size()) ? LENIA_CONV_DIRECT
-                                                                                                      : LENIA_CONV_FFT;
+                    b.path[i] = direct_is_cheaper(taps(i), double(class_members[size_t(cls[i])].size()))
+                                    ? LENIA_CONV_DIRECT
+                                    : LENIA_CONV_FFT;
         }
 
         // Final tables.
@@ -906,7 +928,8 @@ int lenia_batch_step(lenia_batch* bb, uint32_t steps, void* stream) {
         }
         if (steps == 0) return LENIA_OK;
         // The graph for (steps, parity): substeps alternate the parity of the
-        // tables; after each, the device advances seeds and frames.
+        // tables; the device advances seeds and frames (the persistent form after
+        // each, the per-size form once at the end).
         const auto key = std::make_pair(steps, b.cur);
         auto it = b.graphs.find(key);
         if (it == b.graphs.end()) {
