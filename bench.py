@@ -285,7 +285,7 @@ def published_direct_bench(steps: int = 50, warmup: int = 5) -> dict:
     tflops = flops / (ms / 1e3) / 1e12
     return {"workload": "direct, 1 kernel R=32, 1280x720 (the reference's published direct configuration)",
             "ms_per_step": ms, "value": w * h / (ms / 1e3) / 1e6, "unit": UNIT,
-            "direct_tma": info["direct_tma"], "direct_split": info["direct_split"],
+            "tc_engine": info["tc_engine"], "direct_tma": info["direct_tma"], "direct_split": info["direct_split"],
             "direct_outputs_per_thread": info["direct_outputs_per_thread"],
             "direct_rows_per_thread": info["direct_rows_per_thread"],
             "fp32": {"achieved_tflops": tflops, "peak_tflops": peak["ffma_tflops"],

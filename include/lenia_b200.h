@@ -129,12 +129,14 @@ typedef struct lenia_info {
     uint32_t fft_precision;   /* LENIA_FFT_* of the column DFT stages in use */
     uint32_t direct_tma;      /* 1: the direct path loads interior halo tiles by TMA */
     uint32_t direct_split;    /* direct path: thread groups sharing a tile's kernel rows (1, 2, 4, 8) */
-    uint32_t direct_outputs_per_thread; /* direct path: 8, or 16 on large tiles where faster */
+    uint32_t direct_outputs_per_thread; /* direct path: 8, or 16 on large tiles where faster, or in the byte form */
     uint32_t direct_taps;     /* direct path: nonzero kernel taps summed over its kernels */
     uint32_t direct_rows_per_thread; /* direct path: output rows per thread, 1 or 2 (large tiles where faster) */
     uint32_t tc_engine;       /* column DFT stages on the tensor cores: 0 none, 1 mma.sync tiles (radix 16),
                                  2 tcgen05 GEMMs (radix 64, 4096-row fields), 3 the same pipelined over
-                                 two operand slots */
+                                 two operand slots; 4: the direct path's sums as byte products on the
+                                 tensor cores (substeps with a growth centre |mu| < 1/64 run its FP32
+                                 kernels all the same) */
 } lenia_info;
 
 typedef struct lenia_ctx lenia_ctx;

@@ -708,38 +708,41 @@ bool direct_tc_tables(const std::vector<std::vector<float>>& luts, int r, Direct
 
 // Frame times in us as measured back to back on a B200 (148 SMs), one kernel:
 //                      R = 3        5        9        13       20       32
-//   128 x 128   FP32    7.3      8.4      9.1      10.5     13.1     20.9
-//               bytes   9.9     10.5     11.9      13.2     20.7     27.4
-//   512 x 512   FP32    9.0     10.4     13.2      17.3     27.5     62.1
-//               bytes  10.1     10.9     12.1      13.5     21.2     27.8
-//   1001 x 703  FP32   11.1     14.7     25.1      37.2     63.4    133.6
-//               bytes  15.1     15.8     18.5      20.8     32.1     46.3
-//   1280 x 720  FP32   11.3     17.2     29.6      43.9     78.7    183.8
-//               bytes  14.3     14.8     16.1      19.0     30.7     44.8
-//   1920 x 1080 FP32   17.3     25.5     46.0      72.1    134.1    314.5
-//               bytes  21.1     21.8     25.5      29.5     48.1     75.7
+//   128 x 128   FP32    7.2      8.2      8.2      10.2     12.3     20.5
+//               bytes   9.9     10.7     12.4      14.2     22.8     31.6
+//   512 x 512   FP32    8.2     10.2     14.3      16.3     26.6     61.4
+//               bytes  10.2     11.0     12.7      14.5     23.3     32.0
+//   1001 x 703  FP32   12.2     15.3     25.0      38.7     63.5    133.1
+//               bytes  15.2     16.0     19.1      22.6     37.1     55.4
+//   1280 x 720  FP32   11.2     16.4     28.6      43.0     76.5    182.3
+//               bytes  14.3     14.9     17.9      21.5     35.6     53.7
+//   1920 x 1080 FP32   16.6     26.6     45.8      71.6    133.1    311.4
+//               bytes  22.1     22.6     28.0      34.7     59.6     94.8
 // (before the byte form the FP32 column was 205 us at 1280 x 720, R = 32 and 81
-// at 1920 x 1080, R = 13). Both sides are modelled from them: the byte form by
-// its fixed 8.5 us (launch, first tile's staging, last epilogue) and, per round
-// of tiles over the SMs, the larger of the products (87 ns a chunk) and the
-// staging and epilogue (3.4 us); the FP32 form by its 8-tap multiply-adds (3.7e-8
-// us each on fields that fill the SMs evenly, 4.8e-8 below) and 5e-6 us a pixel.
-// A CTA of the byte form holds its SM's tensor memory, so kernels of other
+// at 1920 x 1080, R = 13). Both sides are modelled from them, within 10 % from R
+// = 9 on: the byte form by a fixed 8.3 us (12 above R = 16, whose tiles stage a
+// wider halo: launch, first tile's staging, last epilogue) and, per round of
+// tiles over the SMs, the larger of the products (107 ns a chunk, and 0.9 us to
+// read the sums, which the next products wait for) and the staging and epilogue
+// (3.3 us); the FP32 form by its 8-tap multiply-adds (3.7e-8 us each on fields that
+// fill the SMs evenly, from 2 million pixels on, up to 4.8e-8 below) and 5e-6 us a
+// pixel. A CTA of the byte form holds its SM's tensor memory, so kernels of other
 // contexts fill only the SMs it leaves free: the time a frame costs beside
 // others (its share of the SMs, three quarters of it overlapped at best) counts
 // as much as its own, and its own is at most a tenth longer. Two substeps of
-// 1001 x 703 with noise, jitter and blobs, FP32 / bytes: R = 5 alone 35.2 / 39.2
-// us, beside two others 18.9 / 26.3; R = 9 57.4 / 45.3 and 34.0 / 30.4 us.
+// 1001 x 703, R = 9 with noise, jitter and blobs, FP32 / bytes: alone 56.0 / 50.3
+// us, beside two others 33.8 / 33.8.
 // Kernels of few taps stay on the FP32 form, whose rounding grows with the taps
 // while the byte form's is fixed (they cross at R = 4, 49 taps).
-bool direct_tc_faster(const DirectTcTables& t, uint64_t fp32_taps, int w, int h, int sms) {
+bool direct_tc_faster(const DirectTcTables& t, uint64_t fp32_taps, int r, int w, int h, int sms) {
     if (t.min_taps < 60) return false;
     const double px = double(w) * h;
     const int tiles = ((w + kTX - 1) / kTX) * ((h + kRows - 1) / kRows), rounds = (tiles + sms - 1) / std::max(1, sms);
-    const double bytes = 8.5 + rounds * std::max(0.087 * t.chunks, 3.4);
+    const double bytes = (r <= 16 ? 8.3 : 12.0) + rounds * std::max(0.107 * t.chunks + 0.9, 3.3);
     const double share = 0.75 * bytes * std::min(1.0, double(tiles) / std::max(1, sms));
     const double work = px * (double(fp32_taps) * 3.7e-8 + 5e-6);  // of the FP32 form, the SMs full
-    const double fp32 = 7.0 + px * (double(fp32_taps) * (px < 1.5e6 ? 4.8e-8 : 3.7e-8) + 5e-6);
+    const double tap = 3.7e-8 + 1.1e-8 * std::min(1.0, std::max(0.0, (2.0e6 - px) / 1.1e6));
+    const double fp32 = 7.0 + px * (double(fp32_taps) * tap + 5e-6);
     return bytes + share < fp32 + work && bytes < 1.1 * fp32;
 }
 

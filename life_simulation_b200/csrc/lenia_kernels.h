@@ -85,9 +85,9 @@ struct DirectTcTables {
 // Tables of nk (1..4) kernel tables of (2r + 1)^2 weights; false when they
 // have no byte form (a weight that is not finite, a kernel without weights).
 bool direct_tc_tables(const std::vector<std::vector<float>>& luts, int r, DirectTcTables& out);
-// Whether the tensor-core step is the one to run on a w x h field, against
+// Whether the tensor-core step is the one to run on a w x h field (halo r), against
 // launch_direct_step, which executes fp32_taps multiply-adds a pixel.
-bool direct_tc_faster(const DirectTcTables& t, uint64_t fp32_taps, int w, int h, int sms);
+bool direct_tc_faster(const DirectTcTables& t, uint64_t fp32_taps, int r, int w, int h, int sms);
 // Whether the byte form's sums are as close as the FP32 form's for a substep's
 // growth centres (not for centres near zero, where faint potentials count).
 bool direct_tc_holds(int nk, const StepParams& p);

@@ -664,6 +664,7 @@ int LeniaModule::resolve(uint32_t scene_w, uint32_t scene_h) {
 
 int LeniaModule::setup(uint32_t scene_w, uint32_t scene_h) {
     release();
+    direct_note_.clear();
     const int resolved = resolve(scene_w, scene_h);
     if (resolved < 0) return resolved;
     const std::string warn_msg = message_;
@@ -698,6 +699,10 @@ int LeniaModule::setup(uint32_t scene_w, uint32_t scene_h) {
     spectrum_valid_ = false;
     cur_ = 0;
     message_ = warn_msg;
+    if (!direct_note_.empty()) {
+        message_ += (message_.empty() ? "" : "\n") + direct_note_;
+        return LENIA_WARN_FALLBACK;
+    }
     return resolved;
 }
 
@@ -818,8 +823,12 @@ int LeniaModule::buildDirectTables() {
         uint64_t taps = 0;
         for (uint32_t sp : spans) taps += 8u * (sp >> 16);
         DirectTcTables t;
-        if (want != "ffma" && (want == "tensor" || !shaped) && direct_tc_tables(luts, r, t) &&
-            (want == "tensor" || direct_tc_faster(t, taps, int(w_), int(h_), sms))) {
+        const bool wanted = want != "ffma" && (want == "tensor" || !shaped);
+        const bool held = wanted && direct_tc_tables(luts, r, t);
+        if (want == "tensor" && !held)
+            direct_note_ = "[life] " + instance_ + ": LENIA_DIRECT_ENGINE=tensor: these kernels have no byte form; using "
+                           "the FP32 kernels";
+        if (held && (want == "tensor" || direct_tc_faster(t, taps, r, int(w_), int(h_), sms))) {
             if ((e = dev_alloc(&d_tc_blocks_, t.blocks.size(), device_bytes_)) != cudaSuccess ||
                 (e = dev_alloc(&d_tma_err_, 1, device_bytes_)) != cudaSuccess)
                 return cudaFail(e, "cudaMalloc direct tables");
@@ -828,6 +837,7 @@ int LeniaModule::buildDirectTables() {
             direct_tc_ = t.plan;
             direct_tc_.blocks = d_tc_blocks_;
             direct_tc_on_ = true;
+            // Of the FP32 form, for kernels with mu near zero (direct_tc_holds).
             direct_ox_ = 8;
             direct_oy_ = 1;
             return LENIA_OK;
@@ -950,6 +960,10 @@ int LeniaModule::checkDeviceFlags() {
             return fail(LENIA_ERR_CUDA, "tensor-core column pass: " + std::to_string(n) +
                                             " CTA(s) stopped after a wait for an MMA ran out; their columns were "
                                             "not written");
+        if (direct_tc_on_)
+            return fail(LENIA_ERR_CUDA, "direct path, byte form: " + std::to_string(n) +
+                                            " CTA(s) stopped after a wait ran out; the tiles they had left were not "
+                                            "written");
         return fail(LENIA_ERR_CUDA, "direct path: " + std::to_string(n) +
                                         " halo tile load(s) did not arrive in time; those tiles were not written");
     }
@@ -1456,13 +1470,14 @@ void LeniaModule::info(lenia_info* o) const {
     o->use_stamp_init = use_stamp_ ? 1u : 0u;
     o->device_bytes = device_bytes_;
     o->fft_precision = tc_precision_;
-    o->tc_engine = tc_precision_ == LENIA_FFT_FP32 ? 0u
+    o->tc_engine = !use_fft_ && direct_tc_on_             ? 4u
+                   : tc_precision_ == LENIA_FFT_FP32 ? 0u
                    : tc_batch_ == kTcgen05          ? 2u
                    : tc_batch_ == kTcgen05Pipelined ? 3u
                                                     : 1u;
     o->direct_tma = (!use_fft_ && direct_tma_.on) ? 1u : 0u;
-    o->direct_split = use_fft_ ? 0u : uint32_t(direct_split_);
-    o->direct_outputs_per_thread = use_fft_ ? 0u : uint32_t(direct_ox_);
+    o->direct_split = use_fft_ ? 0u : direct_tc_on_ ? 1u : uint32_t(direct_split_);
+    o->direct_outputs_per_thread = use_fft_ ? 0u : direct_tc_on_ ? 16u : uint32_t(direct_ox_);
     o->direct_rows_per_thread = use_fft_ ? 0u : uint32_t(direct_oy_);
     o->direct_taps = use_fft_ ? 0u : direct_taps_;
     if (use_fft_) {

@@ -202,6 +202,7 @@ private:
     uint32_t* d_spans_ = nullptr;
     // The tensor-core form of the direct step (false: the FP32 kernels run).
     bool direct_tc_on_ = false;
+    std::string direct_note_;  // warning of a forced engine that these kernels cannot take
     DirectTcPlan direct_tc_;
     unsigned char* d_tc_blocks_ = nullptr;
     float* d_org_ = nullptr;
