@@ -136,11 +136,13 @@ __device__ __forceinline__ float bell_fast(float u, float mu, float inv_sigma) {
 // sum_k h_k * (2 bell_k - 1), in kernel order (Lenia.metal:188-195).
 struct EulerStep {
     float dt, sum_weights;
-    bool asym, weighted;
+    bool asym, weighted, divides;
     __device__ __forceinline__ explicit EulerStep(const StepParams& p)
-        : dt(p.dt), sum_weights(p.sum_weights), asym(p.growth_mode == 1u), weighted(p.sum_weights > 1e-6f) {}
-    // dA / dt.
-    __device__ __forceinline__ float rate(float A, float s) const { return asym ? (weighted ? s / sum_weights : A) - A : s; }
+        : dt(p.dt), sum_weights(p.sum_weights), asym(p.growth_mode == 1u), weighted(p.sum_weights > 1e-6f),
+          divides(asym && weighted && p.sum_weights != 1.0f) {}
+    // dA / dt from the sum, divided by the weights' sum where that is not one.
+    __device__ __forceinline__ float rate(float A, float s) const { return rate_of(A, divides ? s / sum_weights : s); }
+    __device__ __forceinline__ float rate_of(float A, float t) const { return asym ? (weighted ? t : A) - A : t; }
     __device__ __forceinline__ float operator()(float A, float s) const { return fmaf(dt, rate(A, s), A); }
     // With its product rounded before the sum: how a batch's direct worlds have always
     // stepped, and over a sweep's thousands of substeps a field amplifies a last place.

@@ -568,12 +568,17 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
                 __syncwarp();
             }
+            if (euler.divides) {  // in a branch of its own: one kernel's weight is one
+#pragma unroll
+                for (int j = 0; j < kPart; ++j) sum[j] = sum[j] / euler.sum_weights;
+            }
             float4* orow = reinterpret_cast<float4*>(dst + size_t(min(gy, H - 1)) * W + gx0);
 #pragma unroll
             for (int c = 0; c < kPart; c += 8) {
                 float v[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) v[j] = euler(av[c + j], sum[c + j]);
+                for (int j = 0; j < 8; ++j)
+                    v[j] = fmaf(euler.dt, euler.rate_of(av[c + j], sum[c + j]), av[c + j]);
                 noise_inject_clip(p, sh.ex, v, uint32_t(gx0 + c), uint32_t(gy));
                 const float4 lo = make_float4(v[0], v[1], v[2], v[3]), hi = make_float4(v[4], v[5], v[6], v[7]);
                 if (!whole) {
