@@ -21,9 +21,9 @@
 // form's own rounding for |mu| >= 2^-6, and kernels nearer zero run on the FP32
 // form (direct_tc_holds). With 24-bit values, rint(a 2^23), a field of 1e-3
 // had a potential off by 6e-5 of itself, two orders above the FP32 form's.
-// An integer sum is the same in any order. A tile whose halo holds a value outside [0, 2)
-// (an uploaded field may: infinities, NaN, negative values) takes the FP32
-// loop below, tap by tap in the order of lenia_direct.cu.
+// An integer sum is the same in any order. A tile whose halo holds a value
+// outside [0, 2) (an uploaded field may: infinities, NaN, negative values) takes
+// the FP32 loop below, tap by tap in the order of lenia_direct.cu.
 //
 // The GEMM. A CTA owns 128 rows x 32 columns of output. Kernel row dy over a
 // chunk of 32 input columns is D[128 x 32] += X[128 x 32] T[32 x 32]: X is the
@@ -196,10 +196,11 @@ __device__ __forceinline__ int wrap(int v, int n) {
     return v < 0 ? v + n : v;
 }
 
-// 0 <= a < 2 exactly when the sign and the top exponent bit are clear (-0
-// takes the FP32 form as well).
+// 0 <= a < 2 exactly when the sign and the top exponent bit are clear; + 0
+// makes -0 zero.
 __device__ __forceinline__ bool out_of_range(const float4& a) {
-    return (((__float_as_uint(a.x) | __float_as_uint(a.y)) | (__float_as_uint(a.z) | __float_as_uint(a.w))) &
+    return (((__float_as_uint(a.x + 0.0f) | __float_as_uint(a.y + 0.0f)) |
+             (__float_as_uint(a.z + 0.0f) | __float_as_uint(a.w + 0.0f))) &
             0xC0000000u) != 0u;
 }
 // Four values as the bytes of levels 0 to 3, value i in byte i.
@@ -214,20 +215,82 @@ __device__ __forceinline__ void pack_bytes(const float4& a, uint32_t (&w)[kPlane
     w[3] = __byte_perm(l01, l23, 0x5410);
 }
 
-// One output of the FP32 form (values the byte form cannot hold): taps in
-// the order of direct_tile.
-__device__ __noinline__ float direct_point(const float* __restrict__ src, const float* __restrict__ weights,
-                                           const uint32_t* __restrict__ spans, const DirectGeometry& g, int W, int H,
-                                           int k, int x, int y) {
-    float acc = 0.0f;
-    for (int dyi = 0; dyi < g.ksize; ++dyi) {
-        const uint32_t sp = spans[k * g.ksize + dyi];
-        const int start = int(sp & 0xFFFFu) - 128, count = int(sp >> 16);
-        const float* row = src + size_t(wrap(y + dyi - g.r, H)) * W;
-        const float* w = weights + size_t(k * g.ksize + dyi) * g.wp + g.xp;
-        for (int d = start; d < start + 8 * count; ++d) acc = fmaf(w[d], row[wrap(x + d, W)], acc);
+// A warp's share of a tile with values that the byte form cannot hold, in the
+// FP32 form: rows y0 .. y0 + 15, a column a lane, taps in the order of
+// direct_tile, four rows at a time on the same weights. Out of line, with no
+// state of the epilogue's alive, so that the tiles of the byte form pay nothing
+// for it. First frames of uploads whose tiles all take it: 1920 x 1080 R = 13
+// 810 us, 1280 x 720 R = 32 1800 us (one output and one tap a thread at a time,
+// rows across the lanes: 7.5 and 19.7 ms; FP32 kernels 104 and 216 us). A step
+// clips its field to [0, 1], so an upload has one such frame.
+constexpr int kFpRows = 16;
+__device__ __noinline__ void fp32_rows(const float* __restrict__ src, float* __restrict__ dst,
+                                       const float* __restrict__ weights, const uint32_t* __restrict__ spans,
+                                       const DirectGeometry& g, const StepParams& p, const GrowthExtras& ex, int nk,
+                                       int x0, int y0) {
+    constexpr int N = 4;
+    const int W = int(p.width), H = int(p.height), x = x0 + int(threadIdx.x & 31u);
+    const EulerStep euler(p);
+#pragma unroll 1
+    for (int y = y0; y < min(y0 + kFpRows, H); y += N) {
+        float sum[N] = {};
+#pragma unroll 1
+        for (int k = 0; k < nk; ++k) {
+            float acc[N] = {};
+#pragma unroll 1
+            for (int dyi = 0; dyi < g.ksize; ++dyi) {
+                const uint32_t sp = spans[k * g.ksize + dyi];
+                const float* w = weights + size_t(k * g.ksize + dyi) * g.wp + g.xp;
+                const float* row[N];
+#pragma unroll
+                for (int j = 0; j < N; ++j) row[j] = src + size_t(wrap(y + j + dyi - g.r, H)) * W;
+                int d = int(sp & 0xFFFFu) - 128;
+#pragma unroll 1
+                for (int c = int(sp >> 16); c > 0; --c, d += 8) {
+                    float a[8][N], t[8];
+                    if (x0 + d >= 0 && x0 + 32 + d + 8 <= W) {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+#pragma unroll
+                            for (int j = 0; j < N; ++j) a[i][j] = __ldg(row[j] + x + d + i);
+                    } else {
+                        int at = wrap(x + d, W);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+#pragma unroll
+                            for (int j = 0; j < N; ++j) a[i][j] = __ldg(row[j] + at);
+                            at = at + 1 == W ? 0 : at + 1;
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) t[i] = __ldg(w + d + i);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+#pragma unroll
+                        for (int j = 0; j < N; ++j) acc[j] = fmaf(t[i], a[i][j], acc[j]);
+                }
+            }
+            const float mu = k == 0 ? p.mu[0] : k == 1 ? p.mu[1] : k == 2 ? p.mu[2] : p.mu[3];
+            const float sigma = k == 0 ? p.sigma[0] : k == 1 ? p.sigma[1] : k == 2 ? p.sigma[2] : p.sigma[3];
+            const float h = k == 0 ? p.weight[0] : k == 1 ? p.weight[1] : k == 2 ? p.weight[2] : p.weight[3];
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                const float shift = p.mu_jitter > 0.0f
+                                        ? mu_jitter_shift(p, uint32_t(x), rand_row(uint32_t(y + j), ex.jitter_base))
+                                        : 0.0f;
+                sum[j] = growth_add(sum[j], h, bell(acc[j], mu + shift, sigma), euler.asym);
+            }
+        }
+#pragma unroll 1
+        for (int j = 0; j < N; ++j) {
+            if (y + j >= H || x >= W) continue;
+            const size_t at = size_t(y + j) * W + size_t(x);
+            const float s = j == 0 ? sum[0] : j == 1 ? sum[1] : j == 2 ? sum[2] : sum[3];
+            float v[1] = {euler(__ldg(src + at), s)};
+            noise_inject_clip(p, ex, v, uint32_t(x), uint32_t(y + j));
+            dst[at] = v[0];
+        }
     }
-    return acc;
 }
 
 // T blocks in flight: what the staged tiles leave room for.
@@ -487,12 +550,13 @@ __global__ void __launch_bounds__(kThreads, 1)
                     av[c] = x < W ? __ldg(src + size_t(min(gq + 2 * c + (lane >> 4), H - 1)) * W + x) : 0.0f;
             }
             float sum[kPart] = {};  // growth sums
+            bool bytes = true;      // no value of the tile's halo outside the byte form
 #pragma unroll 1
             for (int k = 0; k < nk; ++k, ++di) {
                 const uint32_t db = di % kBufs;
                 if (!(ok = bar_wait(&sh.d_full[db], (di / kBufs) & 1u, &sh.stop))) break;
                 fence_after();
-                const bool bytes = *reinterpret_cast<volatile int*>(&sh.bad[ai & 3u]) != int(ai) + 1;
+                bytes = *reinterpret_cast<volatile int*>(&sh.bad[ai & 3u]) != int(ai) + 1;
                 const float scale = pick(plan.scale, k);
                 const float s0 = scale * 512.0f, s1 = scale * 2.0f;
                 const float mu = pick(p.mu, k), sigma = pick(p.sigma, k), weight = pick(p.weight, k);
@@ -535,16 +599,6 @@ __global__ void __launch_bounds__(kThreads, 1)
                 fence_before();
                 __syncwarp();
                 if (lane == 0) bar_arrive(&sh.d_empty[db]);
-                if (!bytes) {
-#pragma unroll 1
-                    for (int j = 0; j < kPart; ++j) {
-                        const float v = gy < H && gx0 + j < W
-                                            ? direct_point(src, weights, spans, g, W, H, k, gx0 + j, gy)
-                                            : 0.0f;
-#pragma unroll
-                        for (int i = 0; i < kPart; ++i) u[i] = i == j ? v : u[i];
-                    }
-                }
 #pragma unroll
                 for (int j = 0; j < kPart / 2; ++j) {
                     const float2 shift = jitter ? mu_jitter_pair(p, sh.ex, uint32_t(gx0 + 2 * j), uint32_t(gy))
@@ -555,6 +609,10 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
             }
             if (!ok) break;  // its tile is left unwritten
+            if (!bytes) {    // for every warp of the tile: the rows are shared out anew
+                fp32_rows(src, dst, weights, spans, g, p, sh.ex, nk, gx0 - kPart * half, gq + kFpRows * half);
+                continue;
+            }
             float* rows = reinterpret_cast<float*>(ring + kStages<P> * kStage) + warp * (32 * kTurn);
             float4* own = reinterpret_cast<float4*>(rows + lane * kTurn);
             if (!whole) {
