@@ -327,8 +327,11 @@ __device__ __forceinline__ void direct_tile(const float* __restrict__ src, float
 #pragma unroll
             for (int k = 0; k < NK; ++k)
                 sum = growth_add(sum, p.weight[k], bell(acc[o][k][j], p.mu[k] + shift, p.sigma[k]), euler.asym);
-            v[j] = BATCH ? euler.rounded(arow[j], sum) : euler(arow[j], sum);
+            v[j] = sum;
         }
+        euler.divide(v);
+#pragma unroll
+        for (int j = 0; j < OX; ++j) v[j] = BATCH ? euler.rounded(arow[j], v[j]) : euler(arow[j], v[j]);
         noise_inject_clip(p, ex, v, uint32_t(x0 + ox), uint32_t(gy));
 #pragma unroll
         for (int j = 0; j < OX; ++j)

@@ -23,8 +23,8 @@
 //     through the growth, into the forward row FFT of A'.
 // Items are mapped with the batch index fastest (lane -> (b, j)), which makes
 // the global loads/stores of the first/last passes contiguous, and shared
-// buffers use a row pitch of 8 banks (mod 32) so lanes of different b do not
-// collide. Complex arithmetic uses the packed FP32x2 instructions.
+// buffers use a row pitch (row_pitch) that keeps lanes of different b on
+// different banks. Complex arithmetic uses the packed FP32x2 instructions.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -409,6 +409,14 @@ __global__ void __launch_bounds__(RowK<PI, RB, SPLIT>::T,
             stage(sA, y0, nk);
             cp_async_wait_all();
             __syncthreads();
+        }
+        // (growth_finish_pair divides by itself)
+        if (nk > 0 && !extras && euler.divides) {  // see EulerStep::divide
+#pragma unroll
+            for (int it = 0; it < K::ITL; ++it)
+#pragma unroll
+                for (int t = 0; t < RC; ++t)
+                    acc[it][t] = make_float2(acc[it][t].x / euler.sum_weights, acc[it][t].y / euler.sum_weights);
         }
         // Euler step, noise, injection, clip (or, with nk == 0, the field as
         // is); the result is kept for the forward row transform (first

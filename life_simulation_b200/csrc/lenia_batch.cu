@@ -18,8 +18,8 @@
 //     last microseconds: 48 worlds of four sizes took 117 us a substep that way
 //     and take 66 us as chains.
 // Either way a CUDA graph captured once replays any number of substeps.
-// Worlds never interact; a world's result is the same as stepping it alone
-// through a single-world context.
+// Worlds never interact; a world's result is the same, bit for bit, as in any
+// other batch that gives it the same path.
 //
 // Path choice (policy AUTO): a world takes the path whose launches cost it
 // less, by a rule on sizes and taps (lenia_batch_create).

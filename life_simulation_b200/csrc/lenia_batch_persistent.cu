@@ -296,7 +296,7 @@ __device__ __noinline__ void row_item(const SpectralWorld& sw, int y0, const flo
                 za[it][t] = a;
                 continue;
             }
-            // A batch's worlds have no noise, mu jitter or injection.
+            // A batch's worlds have no noise, mu jitter or injection, and one kernel of weight one.
             const float2 r = make_float2(fminf(fmaxf(euler(a.x, acc[it][t].x), 0.0f), 1.0f),
                                          fminf(fmaxf(euler(a.y, acc[it][t].y), 0.0f), 1.0f));
             *reinterpret_cast<float2*>(A_out + size_t(gy) * W + 2 * n) = r;

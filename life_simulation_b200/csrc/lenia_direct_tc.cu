@@ -281,6 +281,7 @@ __device__ __noinline__ void fp32_rows(const float* __restrict__ src, float* __r
                 sum[j] = growth_add(sum[j], h, bell(acc[j], mu + shift, sigma), euler.asym);
             }
         }
+        euler.divide(sum);
 #pragma unroll 1
         for (int j = 0; j < N; ++j) {
             if (y + j >= H || x >= W) continue;
@@ -412,33 +413,33 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
             } else {
 #pragma unroll 1
-            for (int i0 = warp - kEpiWarps; i0 < kItems; i0 += kFlight * kStageWarps) {
-                float4 a[kFlight];
+                for (int i0 = warp - kEpiWarps; i0 < kItems; i0 += kFlight * kStageWarps) {
+                    float4 a[kFlight];
 #pragma unroll
-                for (int f = 0; f < kFlight; ++f) {
-                    const int i = i0 + f * kStageWarps, gran = i / kGroups, row = (i - gran * kGroups) * 8 + rl;
-                    const float* line = src + size_t(wrap(y0 - g.r + row, H)) * W;
-                    const int x = x0 - P + 16 * gran + q;
-                    if (inside) {
-                        a[f] = __ldg(reinterpret_cast<const float4*>(line + x));
-                    } else {
-                        a[f].x = __ldg(line + wrap(x, W));
-                        a[f].y = __ldg(line + wrap(x + 1, W));
-                        a[f].z = __ldg(line + wrap(x + 2, W));
-                        a[f].w = __ldg(line + wrap(x + 3, W));
+                    for (int f = 0; f < kFlight; ++f) {
+                        const int i = i0 + f * kStageWarps, gran = i / kGroups, row = (i - gran * kGroups) * 8 + rl;
+                        const float* line = src + size_t(wrap(y0 - g.r + row, H)) * W;
+                        const int x = x0 - P + 16 * gran + q;
+                        if (inside) {
+                            a[f] = __ldg(reinterpret_cast<const float4*>(line + x));
+                        } else {
+                            a[f].x = __ldg(line + wrap(x, W));
+                            a[f].y = __ldg(line + wrap(x + 1, W));
+                            a[f].z = __ldg(line + wrap(x + 2, W));
+                            a[f].w = __ldg(line + wrap(x + 3, W));
+                        }
+                    }
+#pragma unroll
+                    for (int f = 0; f < kFlight; ++f) {
+                        const int i = i0 + f * kStageWarps, gran = i / kGroups, row = (i - gran * kGroups) * 8 + rl;
+                        bad = bad || out_of_range(a[f]);
+                        uint32_t w[kPlanes];
+                        pack_bytes(a[f], w);
+                        unsigned char* o = planes + (gran * RA + row) * 16 + q;
+#pragma unroll
+                        for (int j = 0; j < kPlanes; ++j) *reinterpret_cast<uint32_t*>(o + uint32_t(j) * kPlane) = w[j];
                     }
                 }
-#pragma unroll
-                for (int f = 0; f < kFlight; ++f) {
-                    const int i = i0 + f * kStageWarps, gran = i / kGroups, row = (i - gran * kGroups) * 8 + rl;
-                    bad = bad || out_of_range(a[f]);
-                    uint32_t w[kPlanes];
-                    pack_bytes(a[f], w);
-                    unsigned char* o = planes + (gran * RA + row) * 16 + q;
-#pragma unroll
-                    for (int j = 0; j < kPlanes; ++j) *reinterpret_cast<uint32_t*>(o + uint32_t(j) * kPlane) = w[j];
-                }
-            }
             }
             if (bad) *reinterpret_cast<volatile int*>(&sh.bad[ai & 3u]) = int(ai) + 1;
             asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -626,17 +627,13 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
                 __syncwarp();
             }
-            if (euler.divides) {  // in a branch of its own: one kernel's weight is one
-#pragma unroll
-                for (int j = 0; j < kPart; ++j) sum[j] = sum[j] / euler.sum_weights;
-            }
+            euler.divide(sum);
             float4* orow = reinterpret_cast<float4*>(dst + size_t(min(gy, H - 1)) * W + gx0);
 #pragma unroll
             for (int c = 0; c < kPart; c += 8) {
                 float v[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    v[j] = fmaf(euler.dt, euler.rate_of(av[c + j], sum[c + j]), av[c + j]);
+                for (int j = 0; j < 8; ++j) v[j] = euler(av[c + j], sum[c + j]);
                 noise_inject_clip(p, sh.ex, v, uint32_t(gx0 + c), uint32_t(gy));
                 const float4 lo = make_float4(v[0], v[1], v[2], v[3]), hi = make_float4(v[4], v[5], v[6], v[7]);
                 if (!whole) {
