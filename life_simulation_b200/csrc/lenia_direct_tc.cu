@@ -790,8 +790,8 @@ bool direct_tc_tables(const std::vector<std::vector<float>>& luts, int r, Direct
 // contexts fill only the SMs it leaves free: the time a frame costs beside
 // others (its share of the SMs, three quarters of it overlapped at best) counts
 // as much as its own, and its own is at most a tenth longer. Two substeps of
-// 1001 x 703, R = 9 with noise, jitter and blobs, FP32 / bytes: alone 56.0 / 50.3
-// us, beside two others 33.8 / 33.8.
+// 1001 x 703, R = 9 with noise, jitter and blobs, FP32 / bytes: alone 57.8 / 48.8
+// us, beside two others 33.8 / 32.9.
 // Kernels of few taps stay on the FP32 form, whose rounding grows with the taps
 // while the byte form's is fixed (they cross at R = 4, 49 taps).
 bool direct_tc_faster(const DirectTcTables& t, uint64_t fp32_taps, int r, int w, int h, int sms) {

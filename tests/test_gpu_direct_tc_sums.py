@@ -39,3 +39,26 @@ def test_dense_sums_repeat_and_match_fp64(monkeypatch, kernels, radius):
     # times at 2^-25 of at most 0.35), the growth's slope is dt * 1.22 / sigma = 8.1
     # at most over weights that sum to 1.4, and its exponential and A' round at 2e-7.
     assert np.abs(first - exact).max() <= 1.2e-7 * 8.1 * 1.4 + 2e-7
+
+
+@pytest.mark.parametrize("w,h", [(256, 200), (199, 131)])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_every_option_against_fp64(monkeypatch, w, h, mode):
+    """Noise, mu jitter and blobs on the byte form's epilogue, rows aligned and not."""
+    p = {"convMode": "directMulti", "radius": 14, "growthMode": mode, "kernels": RINGS[:3], "noiseAmount": 0.1,
+         "muJitter": 0.3, "injectAmount": 0.3, "injectCount": 5}
+    a = (np.random.default_rng(w).random((h, w)) * 0.31).astype(np.float32)
+    monkeypatch.setenv("LENIA_DIRECT_ENGINE", "tensor")
+    for f in (0, 13):  # another injection cycle every 12 frames
+        m, o = lb.LeniaModule(p, w, h), OracleLenia(p, w, h, "f64")
+        assert m.info()["tc_engine"] == 4
+        m.reset(9)
+        o.reset(9)
+        m.upload(a)
+        o.set_initial_field(a)
+        m.encode(f, 1)
+        # The sums' and the growth's rounding as above, and 4e-7 a blob and one more
+        # for the noise.
+        assert np.abs(m.field() - o.encode(f, 1)).max() <= 1.2e-7 * 8.1 + 2e-7 + 4e-7 * 6, f
+        m.sync()
+        m.close()
