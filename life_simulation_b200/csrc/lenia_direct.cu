@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 #include <cstring>
 
@@ -71,10 +72,14 @@ cudaError_t launch_t(const float* src, float* dst, const float* weights, const u
                         sizeof(uint32_t) * NK * g.ksize +
                         sizeof(float) * size_t(S - 1) * NK * DirectTile<TW, TH, OX, OY>::kThreads * OX;
     auto fn = direct_step_kernel<TW, TH, NK, S, OX, OY>;
-    // The opt-in of every launch is the same, whatever its radius: two threads
-    // must not lower each other's.
-    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kDirectSmemLimit);
-    if (e != cudaSuccess) return e;
+    // One opt-in whatever the radius: two threads must not lower each other's.
+    static std::atomic<unsigned long long> opted{0};  // context number (see fastfft::prepare)
+    const unsigned long long id = fastfft::context_id();
+    if (id == 0 || opted.load(std::memory_order_acquire) != id) {
+        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kDirectSmemLimit);
+        if (e != cudaSuccess) return e;
+        opted.store(id, std::memory_order_release);
+    }
     CUtensorMap map;
     std::memset(&map, 0, sizeof map);
     const bool on = tma && tma->on && (buffer == 0 || buffer == 1);
